@@ -13,7 +13,10 @@ def _centred(ary, axes, inverse):
         raise ValueError("axes must name two axes")
     t = H.dev(ary)
     if not t.is_complex():
-        t = t.to(K.torch.complex128 if t.dtype != K.torch.float32 else K.torch.complex64)
+        if t.dtype == K.torch.float32:
+            t = t.to(K.torch.complex64)
+        else:  # forward transforms of real data stay real
+            t = t.to(K.torch.complex128 if inverse else K.torch.float64)
     last = [t.ndim - 2, t.ndim - 1]
     moved = axes != last
     if moved:

@@ -1,13 +1,18 @@
 // Image formation (grid2image_spheroid_ms4, standard_grid.py:693-708) and the
 // centred FFT helpers (fft.py:5, ifft.py:5).
 //
-// The ifftshift is a gather in the kernel that fills the cuFFT buffer; the
-// fftshift, the real part, the grid correction 1 / (grdsf(x) grdsf(y)) and
-// the nx*ny / sumwt scaling are one epilogue kernel.  numpy's ifft2 carries
-// 1/(nx*ny), which the reference multiplies back: the unnormalised cuFFT
-// inverse is the same quantity.
+// The image is the real part of the inverse transform, which is the inverse
+// transform of the grid's Hermitian part: k_herm_in gathers it (with the
+// ifftshift) into half-spectrum rows, cuFFT runs Z2D, and k_image_epilogue
+// does the fftshift, the grid correction 1 / (grdsf(x) grdsf(y)) and the
+// nx*ny / sumwt scaling.  numpy's ifft2 carries 1/(nx*ny), which the
+// reference multiplies back: the unnormalised cuFFT inverse is the same
+// quantity.  A real image's forward transform is D2Z, and k_herm_out writes
+// both halves of its spectrum.  Complex data go through Z2Z / C2C
+// (av_fft_shifted).
 #include <cufft.h>
 
+#include <algorithm>
 #include <deque>
 #include <mutex>
 
@@ -16,10 +21,12 @@
 namespace av {
 
 // ----------------------------------------------------------- plan cache ---
+enum FftKind { FFT_C2C, FFT_Z2Z, FFT_Z2D, FFT_D2Z };
+
 struct FftPlan {
   int dev;
   int64_t nplanes, nx, ny;
-  int dbl;
+  FftKind kind;
   cufftHandle h;
   size_t work;
 };
@@ -36,14 +43,19 @@ static std::deque<FftPlan> g_fft_plans;  // stable addresses on push_back
     }                                                                         \
   } while (0)
 
-// Plan for nplanes batched (nx, ny) C2C (Z2Z when dbl) transforms, without
+// Complex columns of a half-spectrum row; a real row in the same buffer is
+// 2 * half_cols doubles apart.
+__host__ __device__ constexpr int64_t half_cols(int64_t ny) { return ny / 2 + 1; }
+
+// Plan for nplanes batched (nx, ny) transforms in place, without
 // auto-allocated work area (the caller's workspace is attached per call).
-static int get_plan(int64_t nplanes, int64_t nx, int64_t ny, int dbl, FftPlan **out) {
+// The real transforms keep ny / 2 + 1 complex (2 (ny / 2 + 1) real) columns.
+static int get_plan(int64_t nplanes, int64_t nx, int64_t ny, FftKind kind, FftPlan **out) {
   int dev = 0;
   AV_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(g_fft_mu);
   for (auto &p : g_fft_plans)
-    if (p.dev == dev && p.nplanes == nplanes && p.nx == nx && p.ny == ny && p.dbl == dbl) {
+    if (p.dev == dev && p.nplanes == nplanes && p.nx == nx && p.ny == ny && p.kind == kind) {
       *out = &p;
       return AV_OK;
     }
@@ -52,13 +64,22 @@ static int get_plan(int64_t nplanes, int64_t nx, int64_t ny, int dbl, FftPlan **
   p.nplanes = nplanes;
   p.nx = nx;
   p.ny = ny;
-  p.dbl = dbl;
+  p.kind = kind;
   AV_CUFFT(cufftCreate(&p.h));
   AV_CUFFT(cufftSetAutoAllocation(p.h, 0));
   long long n[2] = {nx, ny};
   size_t ws = 0;
-  AV_CUFFT(cufftMakePlanMany64(p.h, 2, n, nullptr, 1, nx * ny, nullptr, 1, nx * ny,
-                               dbl ? CUFFT_Z2Z : CUFFT_C2C, nplanes, &ws));
+  if (kind == FFT_Z2D || kind == FFT_D2Z) {
+    const long long h = half_cols(ny);
+    long long cplx[2] = {nx, h}, real[2] = {nx, 2 * h};
+    const bool inv = kind == FFT_Z2D;
+    AV_CUFFT(cufftMakePlanMany64(p.h, 2, n, inv ? cplx : real, 1, nx * (inv ? h : 2 * h),
+                                 inv ? real : cplx, 1, nx * (inv ? 2 * h : h),
+                                 inv ? CUFFT_Z2D : CUFFT_D2Z, nplanes, &ws));
+  } else {
+    AV_CUFFT(cufftMakePlanMany64(p.h, 2, n, nullptr, 1, nx * ny, nullptr, 1, nx * ny,
+                                 kind == FFT_Z2Z ? CUFFT_Z2Z : CUFFT_C2C, nplanes, &ws));
+  }
   p.work = ws;
   g_fft_plans.push_back(p);
   *out = &g_fft_plans.back();
@@ -66,9 +87,9 @@ static int get_plan(int64_t nplanes, int64_t nx, int64_t ny, int dbl, FftPlan **
 }
 
 // Work-area bytes of the (cached) plan for this size.
-static size_t fft_work_bytes(int64_t nplanes, int64_t nx, int64_t ny, int dbl) {
+static size_t fft_work_bytes(int64_t nplanes, int64_t nx, int64_t ny, FftKind kind) {
   FftPlan *p = nullptr;
-  if (get_plan(nplanes, nx, ny, dbl, &p) != AV_OK) return 0;
+  if (get_plan(nplanes, nx, ny, kind, &p) != AV_OK) return 0;
   return p->work;
 }
 
@@ -91,52 +112,213 @@ __global__ void k_ishift_in(const IT *in, CT *buf, int64_t nplanes, int64_t nx, 
   buf[k] = o;
 }
 
-// fftshift of the transform + real part + grid correction + normalisation.
-template <typename CT, typename OT>
-__global__ void k_image_epilogue(const CT *buf, OT *img, const double *sumw, int64_t nplanes,
-                                 int64_t nx, int64_t ny, int apply_corr) {
-  int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  int64_t n = nplanes * nx * ny;
-  if (k >= n) return;
-  int64_t p = k / (nx * ny), r = k - p * nx * ny;
-  int64_t i = r / ny, j = r - i * ny;
-  // fftshift: out[i] = in[(i - nx/2) mod nx] = in[(i + nx - nx/2) % nx]
-  int64_t si = i + (nx - nx / 2);
-  if (si >= nx) si -= nx;
-  int64_t sj = j + (ny - ny / 2);
-  if (sj >= ny) sj -= ny;
-  double v = (double)buf[p * nx * ny + si * ny + sj].x;
-  if (apply_corr) {
-    double cx = (double)(i - nx / 2) / (double)nx;
-    double cy = (double)(j - ny / 2) / (double)ny;
-    double corr = pswf_grdsf(fabs(2.0 * cx)) * pswf_grdsf(fabs(2.0 * cy));
-    v = v / corr;
-  }
-  if (sumw) v = v / sumw[p];
-  img[k] = (OT)v;
+// The kernels around the real transforms.  A block takes IMG_COLS columns of
+// IMG_ROWS rows of one plane (grid: column tiles, row groups, planes), so a
+// thread evaluates the grid correction's factor of its column once and the
+// block the factors of its rows once: an evaluation per pixel, a long chain
+// of FP64 operations and divides, had made the epilogue of four 2048^2 images
+// 548 us (now 85).  IMG_UNROLL rows in flight per thread.  16 rows to a block
+// give a 1024^2 image enough blocks (prologue and epilogue 20 us; 30 with
+// 32 rows), 32 would take four 2048^2 images from 85 to 78.
+// The real transforms themselves halve what the complex ones moved: the
+// gather 95 -> 65 us and cuFFT 289 -> 175 us for four 2048^2 planes, whole
+// images 932 -> 325 us.  Batches of planes small enough to stay in L2 between
+// the passes gained nothing (374 us: cuFFT is bound by its FP64 work there).
+constexpr int IMG_COLS = 128, IMG_ROWS = 16, IMG_UNROLL = 4;
+
+static dim3 img_grid(int64_t nplanes, int64_t rows, int64_t cols) {
+  return dim3((unsigned)((cols + IMG_COLS - 1) / IMG_COLS),
+              (unsigned)std::min<int64_t>((rows + IMG_ROWS - 1) / IMG_ROWS, 65535),
+              (unsigned)std::min<int64_t>(nplanes, 65535));
 }
 
-// Real image -> ifftshift gather into the complex FP64 transform buffer,
-// divided by the grid correction grdsf(x) grdsf(y) when asked.
-template <typename IT>
-__global__ void k_image_prologue(const IT *img, double2 *buf, int64_t nplanes, int64_t nx,
-                                 int64_t ny, int apply_corr) {
-  int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  int64_t n = nplanes * nx * ny;
-  if (k >= n) return;
-  int64_t p = k / (nx * ny), r = k - p * nx * ny;
-  int64_t i = r / ny, j = r - i * ny;
-  int64_t si = i + nx / 2;
-  if (si >= nx) si -= nx;
-  int64_t sj = j + ny / 2;
-  if (sj >= ny) sj -= ny;
-  double v = (double)img[p * nx * ny + si * ny + sj];
-  if (apply_corr) {
-    double cx = (double)(si - nx / 2) / (double)nx;
-    double cy = (double)(sj - ny / 2) / (double)ny;
-    v = v / (pswf_grdsf(fabs(2.0 * cx)) * pswf_grdsf(fabs(2.0 * cy)));
+// i + s for 0 <= i < n, 0 <= s <= n, modulo n.
+__device__ __forceinline__ int64_t wrap(int64_t i, int64_t s, int64_t n) {
+  i += s;
+  return i >= n ? i - n : i;
+}
+
+// Grid-correction factor of pixel i of n along one axis.
+__device__ __forceinline__ double corr_factor(int64_t i, int64_t n) {
+  return pswf_grdsf(fabs(2.0 * ((double)(i - n / 2) / (double)n)));
+}
+
+// v / d for d near 1 / r (a few ulp), Markstein's correction ("Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990): one
+// Newton step makes r the rounded reciprocal, and the exact remainder of
+// v r corrects the quotient's last bit.  7 FP64 operations per pixel in place
+// of a divide's call; zeros, infinities, NaN and results whose remainder
+// could leave the normal range take the divide.
+__device__ __forceinline__ double quotient(double v, double d, double r) {
+  r = fma(r, fma(-d, r, 1.0), r);
+  double q = v * r;
+  const double m = fabs(q);
+  if (!(m > 1e-250 && m < 1e250)) return v / d;
+  return fma(fma(-q, d, v), r, q);
+}
+
+// Calls f(plane, row, column, ...) for every pixel of this block's share,
+// IMG_UNROLL rows at a time: f.load first, then f.store with the grid
+// correction's factors and their reciprocals (1 without apply_corr).
+template <typename F>
+__device__ __forceinline__ void for_pixels(int64_t nplanes, int64_t nx, int64_t ny,
+                                           int apply_corr, F f) {
+  __shared__ double2 s_gx[IMG_ROWS];
+  const int64_t j = blockIdx.x * (int64_t)IMG_COLS + threadIdx.x;
+  double2 gy = make_double2(1.0, 1.0);
+  if (apply_corr && j < ny) {
+    gy.x = corr_factor(j, ny);
+    gy.y = 1.0 / gy.x;
   }
-  buf[k] = make_double2(v, 0.0);
+  for (int64_t i0 = blockIdx.y * (int64_t)IMG_ROWS; i0 < nx;
+       i0 += gridDim.y * (int64_t)IMG_ROWS) {
+    __syncthreads();
+    if (threadIdx.x < IMG_ROWS && i0 + threadIdx.x < nx) {
+      const double g = apply_corr ? corr_factor(i0 + threadIdx.x, nx) : 1.0;
+      s_gx[threadIdx.x] = make_double2(g, 1.0 / g);
+    }
+    __syncthreads();
+    if (j >= ny) continue;
+    const int rows = (int)std::min<int64_t>(IMG_ROWS, nx - i0);
+    for (int64_t p = blockIdx.z; p < nplanes; p += gridDim.z) {
+      const double sw = f.sumw ? f.sumw[p] : 1.0, rsw = 1.0 / sw;
+      for (int r = 0; r < rows; r += IMG_UNROLL) {
+        double v[IMG_UNROLL];
+#pragma unroll
+        for (int k = 0; k < IMG_UNROLL; ++k)
+          if (r + k < rows) v[k] = f.load(p, i0 + r + k, j);
+#pragma unroll
+        for (int k = 0; k < IMG_UNROLL; ++k)
+          if (r + k < rows) f.store(p, i0 + r + k, j, v[k], s_gx[r + k], gy, sw, rsw);
+      }
+    }
+  }
+}
+
+// Half spectrum of the Hermitian part of the ifftshifted grid:
+// buf[i, j] = (s[i, j] + conj(s[-i, -j])) / 2, j <= ny / 2, with
+// s[i, j] = grid[(i + nx/2) % nx, (j + ny/2) % ny].
+template <typename IT>
+__global__ void __launch_bounds__(IMG_COLS) k_herm_in(const IT *grid, double2 *buf,
+                                                      int64_t nplanes, int64_t nx, int64_t ny) {
+  const int64_t h = half_cols(ny);
+  const int64_t j = blockIdx.x * (int64_t)IMG_COLS + threadIdx.x;
+  if (j >= h) return;
+  const int64_t ja = wrap(j, ny / 2, ny);
+  const int64_t jb = wrap(j == 0 ? 0 : ny - j, ny / 2, ny);
+  for (int64_t i0 = blockIdx.y * (int64_t)IMG_ROWS; i0 < nx;
+       i0 += gridDim.y * (int64_t)IMG_ROWS) {
+    const int rows = (int)std::min<int64_t>(IMG_ROWS, nx - i0);
+    for (int64_t p = blockIdx.z; p < nplanes; p += gridDim.z) {
+      const IT *g = grid + p * nx * ny;
+      for (int r = 0; r < rows; r += IMG_UNROLL) {
+        IT a[IMG_UNROLL], b[IMG_UNROLL];
+#pragma unroll
+        for (int k = 0; k < IMG_UNROLL; ++k)
+          if (r + k < rows) {
+            const int64_t i = i0 + r + k;
+            a[k] = __ldcs(g + wrap(i, nx / 2, nx) * ny + ja);
+            b[k] = __ldcs(g + wrap(i == 0 ? 0 : nx - i, nx / 2, nx) * ny + jb);
+          }
+#pragma unroll
+        for (int k = 0; k < IMG_UNROLL; ++k)
+          if (r + k < rows)
+            buf[(p * nx + i0 + r + k) * h + j] =
+                make_double2(0.5 * ((double)a[k].x + (double)b[k].x),
+                             0.5 * ((double)a[k].y - (double)b[k].y));
+      }
+    }
+  }
+}
+
+// fftshift of the transform + grid correction + normalisation:
+// img[i, j] = t[(i + nx - nx/2) % nx, (j + ny - ny/2) % ny] / (gx gy) / sumw.
+template <typename OT>
+struct ImageEpilogue {
+  const double *buf;
+  OT *img;
+  const double *sumw;
+  int64_t nx, ny;
+  int apply_corr;
+  __device__ __forceinline__ double load(int64_t p, int64_t i, int64_t j) const {
+    return buf[(p * nx + wrap(i, nx - nx / 2, nx)) * (2 * half_cols(ny)) +
+               wrap(j, ny - ny / 2, ny)];
+  }
+  __device__ __forceinline__ void store(int64_t p, int64_t i, int64_t j, double v, double2 gx,
+                                        double2 gy, double sw, double rsw) const {
+    if (apply_corr) v = quotient(v, gx.x * gy.x, gx.y * gy.y);
+    if (sumw) v = quotient(v, sw, rsw);
+    __stcs(img + (p * nx + i) * ny + j, (OT)v);
+  }
+};
+
+template <typename OT>
+__global__ void __launch_bounds__(IMG_COLS) k_image_epilogue(ImageEpilogue<OT> f,
+                                                             int64_t nplanes) {
+  for_pixels(nplanes, f.nx, f.ny, f.apply_corr, f);
+}
+
+// ifftshift of a real image into the transform's real rows, divided by the
+// grid correction when asked.
+template <typename IT>
+struct ImagePrologue {
+  const IT *img;
+  double *buf;
+  const double *sumw;  // none
+  int64_t nx, ny;
+  int apply_corr;
+  __device__ __forceinline__ double load(int64_t p, int64_t i, int64_t j) const {
+    return (double)img[(p * nx + i) * ny + j];
+  }
+  __device__ __forceinline__ void store(int64_t p, int64_t i, int64_t j, double v, double2 gx,
+                                        double2 gy, double, double) const {
+    if (apply_corr) v = quotient(v, gx.x * gy.x, gx.y * gy.y);
+    buf[(p * nx + wrap(i, nx - nx / 2, nx)) * (2 * half_cols(ny)) + wrap(j, ny - ny / 2, ny)] =
+        v;
+  }
+};
+
+template <typename IT>
+__global__ void __launch_bounds__(IMG_COLS) k_image_prologue(ImagePrologue<IT> f,
+                                                             int64_t nplanes) {
+  for_pixels(nplanes, f.nx, f.ny, f.apply_corr, f);
+}
+
+// fftshift of a half spectrum to a full grid: the other half is the
+// conjugate of the mirrored one.
+template <typename OT>
+__global__ void __launch_bounds__(IMG_COLS) k_herm_out(const double2 *buf, OT *grid,
+                                                       int64_t nplanes, int64_t nx,
+                                                       int64_t ny) {
+  const int64_t h = half_cols(ny);
+  const int64_t j = blockIdx.x * (int64_t)IMG_COLS + threadIdx.x;
+  if (j >= ny) return;
+  const int64_t sj = wrap(j, ny - ny / 2, ny);
+  const bool mirror = sj >= h;
+  const int64_t bj = mirror ? ny - sj : sj;
+  for (int64_t i0 = blockIdx.y * (int64_t)IMG_ROWS; i0 < nx;
+       i0 += gridDim.y * (int64_t)IMG_ROWS) {
+    const int rows = (int)std::min<int64_t>(IMG_ROWS, nx - i0);
+    for (int64_t p = blockIdx.z; p < nplanes; p += gridDim.z)
+      for (int r = 0; r < rows; r += IMG_UNROLL) {
+        double2 v[IMG_UNROLL];
+#pragma unroll
+        for (int k = 0; k < IMG_UNROLL; ++k)
+          if (r + k < rows) {
+            int64_t si = wrap(i0 + r + k, nx - nx / 2, nx);
+            if (mirror && si != 0) si = nx - si;
+            v[k] = buf[(p * nx + si) * h + bj];
+          }
+#pragma unroll
+        for (int k = 0; k < IMG_UNROLL; ++k)
+          if (r + k < rows) {
+            OT o;
+            o.x = v[k].x;
+            o.y = mirror ? -v[k].y : v[k].y;
+            grid[(p * nx + i0 + r + k) * ny + j] = o;
+          }
+      }
+  }
 }
 
 // fftshift gather of a complex result: out[i] = buf[(i + nx - nx/2) % nx].
@@ -159,17 +341,39 @@ __global__ void k_shift_out(const CT *buf, OT *out, int64_t nplanes, int64_t nx,
   out[k] = o;
 }
 
-static int run_fft(void *buf, int dbl, int64_t nplanes, int64_t nx, int64_t ny, int dir,
+// In place on buf; dir counts for the complex kinds.
+static int run_fft(void *buf, FftKind kind, int64_t nplanes, int64_t nx, int64_t ny, int dir,
                    void *work, cudaStream_t st) {
   FftPlan *p = nullptr;
-  int rc = get_plan(nplanes, nx, ny, dbl, &p);
+  int rc = get_plan(nplanes, nx, ny, kind, &p);
   if (rc) return rc;
   AV_CUFFT(cufftSetStream(p->h, st));
   AV_CUFFT(cufftSetWorkArea(p->h, work));
-  if (dbl)
-    AV_CUFFT(cufftExecZ2Z(p->h, (cufftDoubleComplex *)buf, (cufftDoubleComplex *)buf, dir));
-  else
-    AV_CUFFT(cufftExecC2C(p->h, (cufftComplex *)buf, (cufftComplex *)buf, dir));
+  switch (kind) {
+    case FFT_C2C:
+      AV_CUFFT(cufftExecC2C(p->h, (cufftComplex *)buf, (cufftComplex *)buf, dir));
+      break;
+    case FFT_Z2Z:
+      AV_CUFFT(cufftExecZ2Z(p->h, (cufftDoubleComplex *)buf, (cufftDoubleComplex *)buf, dir));
+      break;
+    case FFT_Z2D:
+      AV_CUFFT(cufftExecZ2D(p->h, (cufftDoubleComplex *)buf, (cufftDoubleReal *)buf));
+      break;
+    case FFT_D2Z:
+      AV_CUFFT(cufftExecD2Z(p->h, (cufftDoubleReal *)buf, (cufftDoubleComplex *)buf));
+      break;
+  }
+  return AV_OK;
+}
+
+// Buffer and work area of a real transform of nplanes planes.
+static int real_fft_need(int64_t nplanes, int64_t nx, int64_t ny, FftKind kind, size_t *buf,
+                         size_t *work) {
+  *buf = (size_t)nplanes * nx * half_cols(ny) * 16;
+  FftPlan *p = nullptr;
+  int rc = get_plan(nplanes, nx, ny, kind, &p);
+  if (rc) return rc;
+  *work = p->work;
   return AV_OK;
 }
 
@@ -182,15 +386,20 @@ extern "C" {
 size_t av_fft_workspace_size(int64_t nplanes, int64_t nx, int64_t ny, int precision) {
   int dbl = precision == AV_F64 || precision == AV_C128;
   size_t buf = (size_t)nplanes * nx * ny * (dbl ? 16 : 8);
-  return Workspace::need(buf) + Workspace::need(fft_work_bytes(nplanes, nx, ny, dbl));
+  return Workspace::need(buf) +
+         Workspace::need(fft_work_bytes(nplanes, nx, ny, dbl ? FFT_Z2Z : FFT_C2C));
 }
 
 size_t av_grid_to_image_workspace_size(int64_t nplanes, int64_t nx, int64_t ny) {
-  size_t buf = (size_t)nplanes * nx * ny * 16;
-  return Workspace::need(buf) + Workspace::need(fft_work_bytes(nplanes, nx, ny, 1));
+  // av_image_to_grid takes the same workspace
+  size_t buf = 0, inv = 0, fwd = 0;
+  if (nplanes <= 0 || nx <= 0 || ny <= 0) return 0;
+  real_fft_need(nplanes, nx, ny, FFT_Z2D, &buf, &inv);
+  real_fft_need(nplanes, nx, ny, FFT_D2Z, &buf, &fwd);
+  return Workspace::need(buf) + Workspace::need(std::max(inv, fwd));
 }
 
-// The transform is always FP64 (Z2Z): the grid correction divides by a taper
+// The transform is always FP64: the grid correction divides by a taper
 // that is ~4e-3 at the image edges, which would amplify FP32 transform
 // rounding to ~1e-4 relative error in the image.
 int av_grid_to_image(const void *grid, int grid_dtype, const double *sum_weight, void *image,
@@ -202,36 +411,36 @@ int av_grid_to_image(const void *grid, int grid_dtype, const double *sum_weight,
   AV_CHECK_ARG(image_dtype == AV_F32 || image_dtype == AV_F64, "av_grid_to_image: image dtype");
   AV_CHECK_ARG(nplanes >= 0 && nx > 0 && ny > 0, "av_grid_to_image: bad shape");
   if (nplanes == 0) return AV_OK;
-  FftPlan *p = nullptr;
-  int rc = get_plan(nplanes, nx, ny, 1, &p);
+  size_t bufb = 0, workb = 0;
+  int rc = real_fft_need(nplanes, nx, ny, FFT_Z2D, &bufb, &workb);
   if (rc) return rc;
-  size_t bufb = (size_t)nplanes * nx * ny * 16;
-  if (!workspace || workspace_bytes < Workspace::need(bufb) + Workspace::need(p->work)) {
+  if (!workspace || workspace_bytes < Workspace::need(bufb) + Workspace::need(workb)) {
     set_error("av_grid_to_image: workspace too small (%zu < %zu)", workspace_bytes,
-              Workspace::need(bufb) + Workspace::need(p->work));
+              Workspace::need(bufb) + Workspace::need(workb));
     return AV_ERR_WORKSPACE;
   }
   Workspace ws(workspace, workspace_bytes);
-  double2 *buf = ws.take<double2>((size_t)nplanes * nx * ny);
-  void *work = ws.take<char>(p->work > 0 ? p->work : 1);
+  double2 *buf = ws.take<double2>(bufb / sizeof(double2));
+  void *work = ws.take<char>(workb > 0 ? workb : 1);
   cudaStream_t st = as_stream(stream);
-  int64_t n = nplanes * nx * ny;
-  unsigned blocks = (unsigned)((n + 255) / 256);
+  const dim3 half = img_grid(nplanes, nx, half_cols(ny)), full = img_grid(nplanes, nx, ny);
   if (grid_dtype == AV_C128)
-    k_ishift_in<double2, double2><<<blocks, 256, 0, st>>>((const double2 *)grid, buf, nplanes,
-                                                         nx, ny);
+    k_herm_in<double2><<<half, IMG_COLS, 0, st>>>((const double2 *)grid, buf, nplanes,
+                                                  nx, ny);
   else
-    k_ishift_in<double2, float2><<<blocks, 256, 0, st>>>((const float2 *)grid, buf, nplanes, nx,
-                                                        ny);
+    k_herm_in<float2><<<half, IMG_COLS, 0, st>>>((const float2 *)grid, buf, nplanes, nx,
+                                                 ny);
   AV_LAUNCH_CHECK();
-  rc = run_fft(buf, 1, nplanes, nx, ny, CUFFT_INVERSE, work, st);
+  rc = run_fft(buf, FFT_Z2D, nplanes, nx, ny, CUFFT_INVERSE, work, st);
   if (rc) return rc;
   if (image_dtype == AV_F64)
-    k_image_epilogue<double2, double><<<blocks, 256, 0, st>>>(buf, (double *)image, sum_weight,
-                                                             nplanes, nx, ny, apply_corr);
+    k_image_epilogue<double><<<full, IMG_COLS, 0, st>>>(
+        ImageEpilogue<double>{(const double *)buf, (double *)image, sum_weight, nx, ny,
+                              apply_corr}, nplanes);
   else
-    k_image_epilogue<double2, float><<<blocks, 256, 0, st>>>(buf, (float *)image, sum_weight,
-                                                            nplanes, nx, ny, apply_corr);
+    k_image_epilogue<float><<<full, IMG_COLS, 0, st>>>(
+        ImageEpilogue<float>{(const double *)buf, (float *)image, sum_weight, nx, ny,
+                             apply_corr}, nplanes);
   AV_LAUNCH_CHECK();
   return AV_OK;
 }
@@ -248,35 +457,34 @@ int av_image_to_grid(const void *image, int image_dtype, void *grid, int grid_dt
   AV_CHECK_ARG(grid_dtype == AV_C64 || grid_dtype == AV_C128, "av_image_to_grid: grid dtype");
   AV_CHECK_ARG(nplanes >= 0 && nx > 0 && ny > 0, "av_image_to_grid: bad shape");
   if (nplanes == 0) return AV_OK;
-  FftPlan *p = nullptr;
-  int rc = get_plan(nplanes, nx, ny, 1, &p);
+  size_t bufb = 0, workb = 0;
+  int rc = real_fft_need(nplanes, nx, ny, FFT_D2Z, &bufb, &workb);
   if (rc) return rc;
-  size_t bufb = (size_t)nplanes * nx * ny * 16;
-  if (!workspace || workspace_bytes < Workspace::need(bufb) + Workspace::need(p->work)) {
+  if (!workspace || workspace_bytes < Workspace::need(bufb) + Workspace::need(workb)) {
     set_error("av_image_to_grid: workspace too small");
     return AV_ERR_WORKSPACE;
   }
   Workspace ws(workspace, workspace_bytes);
-  double2 *buf = ws.take<double2>((size_t)nplanes * nx * ny);
-  void *work = ws.take<char>(p->work > 0 ? p->work : 1);
+  double2 *buf = ws.take<double2>(bufb / sizeof(double2));
+  void *work = ws.take<char>(workb > 0 ? workb : 1);
   cudaStream_t st = as_stream(stream);
-  int64_t n = nplanes * nx * ny;
-  unsigned blocks = (unsigned)((n + 255) / 256);
+  const dim3 full = img_grid(nplanes, nx, ny);
   if (image_dtype == AV_F64)
-    k_image_prologue<double><<<blocks, 256, 0, st>>>((const double *)image, buf, nplanes, nx, ny,
-                                                     apply_corr);
+    k_image_prologue<double><<<full, IMG_COLS, 0, st>>>(
+        ImagePrologue<double>{(const double *)image, (double *)buf, nullptr, nx, ny,
+                              apply_corr}, nplanes);
   else
-    k_image_prologue<float><<<blocks, 256, 0, st>>>((const float *)image, buf, nplanes, nx, ny,
-                                                    apply_corr);
+    k_image_prologue<float><<<full, IMG_COLS, 0, st>>>(
+        ImagePrologue<float>{(const float *)image, (double *)buf, nullptr, nx, ny,
+                             apply_corr}, nplanes);
   AV_LAUNCH_CHECK();
-  rc = run_fft(buf, 1, nplanes, nx, ny, CUFFT_FORWARD, work, st);
+  rc = run_fft(buf, FFT_D2Z, nplanes, nx, ny, CUFFT_FORWARD, work, st);
   if (rc) return rc;
   if (grid_dtype == AV_C128)
-    k_shift_out<double2, double2><<<blocks, 256, 0, st>>>(buf, (double2 *)grid, nplanes, nx, ny,
-                                                         1.0);
+    k_herm_out<double2><<<full, IMG_COLS, 0, st>>>(buf, (double2 *)grid, nplanes, nx,
+                                                   ny);
   else
-    k_shift_out<double2, float2><<<blocks, 256, 0, st>>>(buf, (float2 *)grid, nplanes, nx, ny,
-                                                        1.0);
+    k_herm_out<float2><<<full, IMG_COLS, 0, st>>>(buf, (float2 *)grid, nplanes, nx, ny);
   AV_LAUNCH_CHECK();
   return AV_OK;
 }
@@ -289,8 +497,9 @@ int av_fft_shifted(const void *in, void *out, int dtype, int64_t nplanes, int64_
   AV_CHECK_ARG(nplanes >= 0 && nx > 0 && ny > 0, "av_fft_shifted: bad shape");
   if (nplanes == 0) return AV_OK;
   int dbl = dtype == AV_C128;
+  const FftKind kind = dbl ? FFT_Z2Z : FFT_C2C;
   FftPlan *p = nullptr;
-  int rc = get_plan(nplanes, nx, ny, dbl, &p);
+  int rc = get_plan(nplanes, nx, ny, kind, &p);
   if (rc) return rc;
   size_t bufb = (size_t)nplanes * nx * ny * (dbl ? 16 : 8);
   if (!workspace || workspace_bytes < Workspace::need(bufb) + Workspace::need(p->work)) {
@@ -311,7 +520,7 @@ int av_fft_shifted(const void *in, void *out, int dtype, int64_t nplanes, int64_
     k_ishift_in<float2, float2><<<blocks, 256, 0, st>>>((const float2 *)in, (float2 *)buf,
                                                        nplanes, nx, ny);
   AV_LAUNCH_CHECK();
-  rc = run_fft(buf, dbl, nplanes, nx, ny, inverse ? CUFFT_INVERSE : CUFFT_FORWARD, work, st);
+  rc = run_fft(buf, kind, nplanes, nx, ny, inverse ? CUFFT_INVERSE : CUFFT_FORWARD, work, st);
   if (rc) return rc;
   if (dbl)
     k_shift_out<double2, double2><<<blocks, 256, 0, st>>>((const double2 *)buf, (double2 *)out,

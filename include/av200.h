@@ -370,7 +370,8 @@ size_t av_fft_workspace_size(int64_t nplanes, int64_t nx, int64_t ny, int precis
 /* grid2image_spheroid_ms4's image step, standard_grid.py:693-708:
  * image[p] = Re(fftshift(ifft2(ifftshift(grid[p])))) / corrTerm * nx*ny /
  * sum_weight[p] for nplanes planes of (nx, ny).  grid AV_C64 or AV_C128;
- * the transform is always an FP64 cuFFT Z2Z; image AV_F32 or AV_F64.
+ * the transform is always FP64 (cuFFT Z2D of the grid's Hermitian part, whose
+ * transform is the real part); image AV_F32 or AV_F64.
  * sum_weight may be NULL (no division). apply_corr = 0 skips corrTerm. */
 size_t av_grid_to_image_workspace_size(int64_t nplanes, int64_t nx, int64_t ny);
 int av_grid_to_image(const void *grid, int grid_dtype, const double *sum_weight,
