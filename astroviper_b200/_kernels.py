@@ -110,6 +110,37 @@ def degrid_tiled_ok(precision, support, sampling, g_npol, c):
             and float(c) == C_LIGHT)
 
 
+def _plan_us(rows, planes, nu, nv, support):
+    """Microseconds a binning plan costs (ten launches, 8 ps a cell key for its
+    scan, 50 ps a sample)."""
+    tiles = planes * (-(-(nu - support + 1) // 32)) * (-(-(nv - support + 1) // 32))
+    return 40.0 + 8e-6 * 1024 * tiles + 5e-5 * rows
+
+
+def _binning_pays(plain_ps, rows, npol, planes, nu, nv, support):
+    """Whether binning the samples first beats the plain FP64 kernel, which
+    takes plain_ps picoseconds a tap and correlation (33 for the gridder, 2.5
+    for the degridder, 806k samples x 2 pol, support 7: 2620 and 199 us, binned
+    109 and 128 us with the plan).  The binned kernels' own time hides behind
+    the plan's.  The plan also has to fit its key and row ranges."""
+    if (not 3 <= support <= 9 or nu < support or nv < support or max(nu, nv) >= 131072
+            or rows >= 1 << 31):
+        return False
+    tiles = planes * (-(-(nu - support + 1) // 32)) * (-(-(nv - support + 1) // 32))
+    if tiles * 1024 > (1 << 28) - 65536:
+        return False
+    plain = plain_ps * 1e-6 * rows * npol * support * support
+    return plain > _plan_us(rows, planes, nu, nv, support)
+
+
+def _scratch(nbytes):
+    """workspace(), or None when the device has no room for it."""
+    try:
+        return workspace(nbytes)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def grid(vis, weight, uvw, freq, chan_map, pol_map, cgk, n_uv, delta_lm, support,
          oversampling, n_img_chan, n_img_pol, grid_out=None, sum_weight=None, do_psf=False,
          do_imaging_weight=False, precision="fp32"):
@@ -143,6 +174,21 @@ def grid(vis, weight, uvw, freq, chan_map, pol_map, cgk, n_uv, delta_lm, support
         v = None if do_psf else on_device(vis)
         if v is not None and v.dtype not in (torch.complex64, torch.complex128):
             v = v.to(torch.complex128)
+        if (grid_tiled_ok("fp32", do_imaging_weight, support, oversampling, npol, n_img_pol)
+                and grid_out.is_complex()
+                and cgk.numel() >= int(oversampling) * (int(support) // 2 + 1)
+                and _binning_pays(33.0, nt * nb * nchan, npol, int(n_img_chan), nu, nv,
+                                  int(support))):
+            ws = _scratch(lib().av_grid_tiled_workspace_size(nt, nb, nchan, nu, nv,
+                                                             int(n_img_chan), int(support)))
+            if ws is not None:
+                check(lib().av_grid_double(
+                    p(grid_out), dcode(grid_out), p(sum_weight), int(bool(do_psf)), p(v),
+                    dcode(v) if v is not None else AV_C128, p(w), dcode(w), p(uvw), p(freq),
+                    p(cm), p(pm), p(cgk), nu, nv, float(delta_lm[0]), float(delta_lm[1]),
+                    int(support), int(oversampling), nt, nb, nchan, npol, int(n_img_chan),
+                    int(n_img_pol), ws[1], ws[2], stream_ptr()), "av_grid_double")
+                return grid_out, sum_weight
         rc = lib().av_grid_plain(
             p(grid_out), dcode(grid_out), p(sum_weight), int(bool(do_psf)),
             int(bool(do_imaging_weight)), p(v), dcode(v) if v is not None else AV_C128, p(w),
@@ -198,6 +244,20 @@ def degrid(grid_t, uvw, freq, scale, offset, chanmap, polmap, cgk, support, samp
     if not tiled_ok:
         if not accumulate:
             values.zero_()
+        if (degrid_tiled_ok("fp32", support, sampling, g_npol, c) and nvpol <= 4
+                and cgk.numel() >= int(sampling) * (int(support) // 2 + 1)
+                and _binning_pays(2.5, nt * nb * nvchan, nvpol, g_nchan, g_n2, g_n3,
+                                  int(support))):
+            ws = _scratch(lib().av_degrid_tiled_workspace_size(nt, nb, nvchan, g_n2, g_n3,
+                                                               g_nchan, int(support)))
+            if ws is not None:
+                check(lib().av_degrid_double(
+                    p(uvw), p(dph), p(values), dcode(values), p(fl), float(scale[0]),
+                    float(scale[1]), float(offset[0]), float(offset[1]), p(g), dcode(g), g_nchan,
+                    g_npol, g_n2, g_n3, p(freq), int(support), int(sampling), p(cgk), p(cm),
+                    p(pm), nt, nb, nvchan, nvpol, ws[1], ws[2], stream_ptr()),
+                    "av_degrid_double")
+                return values
         args_common = (p(uvw), p(dph), p(values), dcode(values), p(fl), float(scale[0]),
                        float(scale[1]), float(offset[0]), float(offset[1]))
         rc = lib().av_degrid_plain(*args_common, p(g), dcode(g), g_nchan, g_npol, g_n2, g_n3,

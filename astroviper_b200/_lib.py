@@ -65,6 +65,12 @@ SIGNATURES = {
     "av_grid_tiled": (_i, [_vp, _i, _vp, _i, _vp, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i64,
                            _i64, _d, _d, _i, _i, _i64, _i64, _i64, _i64, _i64, _i64, _vp, _sz,
                            _vp]),
+    "av_grid_double": (_i, [_vp, _i, _vp, _i, _vp, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i64,
+                            _i64, _d, _d, _i, _i, _i64, _i64, _i64, _i64, _i64, _i64, _vp, _sz,
+                            _vp]),
+    "av_degrid_double": (_i, [_vp, _vp, _vp, _i, _vp, _d, _d, _d, _d, _vp, _i, _i64, _i64, _i64,
+                              _i64, _vp, _i, _i, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp,
+                              _sz, _vp]),
     "av_degrid_plain": (_i, [_vp, _vp, _vp, _i, _vp, _d, _d, _d, _d, _vp, _i, _i64, _i64, _i64,
                              _i64, _vp, _d, _i, _i, _vp, _vp, _vp, _i64, _i64, _i64, _i64,
                              _vp]),

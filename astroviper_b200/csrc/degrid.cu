@@ -1427,6 +1427,125 @@ __global__ void __launch_bounds__(128) k_degrid_exceptions(ExcArgs e) {
   }
 }
 
+// ---------------------------------------------------- double precision ----
+// k_degrid_plain over a degridder plan: one thread per sorted record, the
+// reference's taps, products and order of summation, so the values are
+// bit-identical to the plain kernel's.  There, neighbouring threads (channels
+// of one baseline) read footprints far apart, 1 KB of L2 traffic per
+// correlation; here a warp's records share a cell or two, every load of the
+// grid is a broadcast from L1, and the taps are formed once for all
+// polarisations.  The small array with 8 channels and
+// 2 polarisations (806k samples): 97 us + 31 us of plan against 199 us.
+struct SortedDegridArgs {
+  const Rec *recs;
+  const uint32_t *tile_start, *n_rec;
+  int64_t n_tiles, ntu, ntv;
+  int cf_len;
+  DegridArgs d;
+};
+
+constexpr int SD_THREADS = 128;
+
+template <int S, int NP>
+__global__ void __launch_bounds__(SD_THREADS) k_degrid_sorted(SortedDegridArgs a) {
+  extern __shared__ double s_cf[];
+  const DegridArgs &d = a.d;
+  for (int i0 = 0; i0 < a.cf_len; i0 += SD_THREADS) {
+    const int i = i0 + threadIdx.x;
+    if (i < a.cf_len) s_cf[i] = d.cf[i];
+  }
+  __syncthreads();
+  const uint32_t n = *a.n_rec;
+  const uint32_t r = blockIdx.x * SD_THREADS + threadIdx.x, w0 = r & ~31u;
+  if (w0 >= n) return;  // the whole warp
+  int64_t t = find_tile_warp(a.tile_start, a.n_tiles, w0);
+  if (r >= n) return;
+  while (a.tile_start[t + 1] <= r) ++t;  // r < n = tile_start[n_tiles]
+  const Rec rc = a.recs[r];
+  const int64_t plane = t / (a.ntu * a.ntv), rest = t - plane * a.ntu * a.ntv;
+  const int64_t fu = (rest / a.ntv) * TILE + rc.du, fv = (rest % a.ntv) * TILE + rc.dv;
+  const int o0 = (int)rc.ou - 128, o1 = (int)rc.ov - 128;
+  const int64_t cells = d.g_n2 * d.g_n3;
+  const int64_t at = plane * d.g_npol * cells + fu * d.g_n3 + fv;
+  double wty[S];
+#pragma unroll
+  for (int j = 0; j < S; ++j) {
+    const int k = d.sampling * (j - S / 2) + o1;
+    wty[j] = s_cf[k < 0 ? -k : k];
+  }
+  int64_t off[NP];
+  unsigned use = 0;  // polarisations to write
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    const int q = p < d.nvpol ? d.polmap[p] : -1;
+    const bool mapped = q >= 0 && q < d.g_npol;
+    off[p] = mapped ? q * cells : 0;
+    if (mapped && !(d.flag && d.flag[(int64_t)rc.row * d.nvpol + p])) use |= 1u << p;
+  }
+  double re[NP], im[NP], norm = 0.0;
+#pragma unroll
+  for (int p = 0; p < NP; ++p) re[p] = im[p] = 0.0;
+#pragma unroll
+  for (int i = 0; i < S; ++i) {
+    const int k = d.sampling * (i - S / 2) + o0;
+    const double wtx = s_cf[k < 0 ? -k : k];
+    const int64_t row = at + i * d.g_n3;
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const double wt = __dmul_rn(wtx, wty[j]);
+      norm = __dadd_rn(norm, wt);
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        double2 g;
+        if (d.grid_c128) {
+          g = __ldg((const double2 *)d.grid + off[p] + row + j);
+        } else {
+          const float2 x = __ldg((const float2 *)d.grid + off[p] + row + j);
+          g = make_double2(x.x, x.y);
+        }
+        re[p] = __dadd_rn(re[p], __dmul_rn(wt, g.x));
+        im[p] = __dadd_rn(im[p], __dmul_rn(wt, g.y));
+      }
+    }
+  }
+  if (norm == 0.0) return;
+  const uint32_t tb = rc.row / (uint32_t)d.nvchan, c = rc.row - tb * (uint32_t)d.nvchan;
+  const double phase = __ddiv_rn(
+      __dmul_rn(__dmul_rn(-2.0 * 3.141592653589793, d.dphase ? d.dphase[tb] : 0.0), d.freq[c]),
+      d.c);
+  double cr = 1.0, ph_im = phase;  // sin(+-0) = +-0
+  if (d.dphase) sincos(phase, &ph_im, &cr);
+  const double ci = -ph_im;
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    if (!((use >> p) & 1u)) continue;
+    const double pr = __dsub_rn(__dmul_rn(re[p], cr), __dmul_rn(im[p], ci));
+    const double pi = __dadd_rn(__dmul_rn(re[p], ci), __dmul_rn(im[p], cr));
+    const double vr = __ddiv_rn(pr, norm), vi = __ddiv_rn(pi, norm);
+    const int64_t k = (int64_t)rc.row * d.nvpol + p;
+    if (d.values_c128) {
+      double2 *o = (double2 *)d.values + k;
+      const double2 cur = *o;
+      *o = make_double2(__dadd_rn(cur.x, vr), __dadd_rn(cur.y, vi));
+    } else {
+      float2 *o = (float2 *)d.values + k;
+      const float2 cur = *o;
+      *o = make_float2((float)((double)cur.x + vr), (float)((double)cur.y + vi));
+    }
+  }
+}
+
+template <int S>
+static int launch_degrid_sorted(const SortedDegridArgs &a, int64_t rows, cudaStream_t st) {
+  const unsigned blocks = (unsigned)((rows + SD_THREADS - 1) / SD_THREADS);
+  const size_t smem = (size_t)a.cf_len * sizeof(double);
+  if (a.d.nvpol <= 1) k_degrid_sorted<S, 1><<<blocks, SD_THREADS, smem, st>>>(a);
+  else if (a.d.nvpol <= 2) k_degrid_sorted<S, 2><<<blocks, SD_THREADS, smem, st>>>(a);
+  else k_degrid_sorted<S, 4><<<blocks, SD_THREADS, smem, st>>>(a);
+  AV_LAUNCH_CHECK();
+  return AV_OK;
+}
+
 template <int S>
 static int launch_degrid_tc(const TiledDegridArgs &a, int64_t nblocks, cudaStream_t st) {
   size_t smem = TCSmem<S>::total;
@@ -1779,6 +1898,51 @@ int av_degrid_tiled(const double *uvw, const double *dphase, void *values, int v
                                  g_nchan,
                                  g_npol, g_n2, g_n3, freq, support, sampling, convFunc, polmap, nt,
                                  nb, nvchan, nvpol, workspace, workspace_bytes, stream);
+}
+
+int av_degrid_double(const double *uvw, const double *dphase, void *values, int values_dtype,
+                     const uint8_t *flag, double scale_x, double scale_y, double offset_x,
+                     double offset_y, const void *grid, int grid_dtype, int64_t g_nchan,
+                     int64_t g_npol, int64_t g_n2, int64_t g_n3, const double *freq, int support,
+                     int sampling, const double *convFunc, const int32_t *chanmap,
+                     const int32_t *polmap, int64_t nt, int64_t nb, int64_t nvchan,
+                     int64_t nvpol, void *workspace, size_t workspace_bytes, void *stream) {
+  clear_error();
+  SortedDegridArgs a;
+  int rc = fill_degrid_args(a.d, uvw, dphase, values, values_dtype, flag, scale_x, scale_y,
+                            offset_x, offset_y, grid, grid_dtype, g_nchan, g_npol, g_n2, g_n3,
+                            freq, C_LIGHT, support, sampling, convFunc, chanmap, polmap, nt, nb,
+                            nvchan, nvpol, "av_degrid_double");
+  if (rc) return rc;
+  AV_CHECK_ARG(nvpol <= 4 && g_npol >= 1,
+               "av_degrid_double: at most 4 visibility polarisations, at least 1 in the grid");
+  PlanGeom g;
+  Plan p;
+  rc = degrid_geom_checked(g, p, scale_x, scale_y, offset_x, offset_y, g_nchan, g_n2, g_n3,
+                           support, sampling, nt, nb, nvchan, workspace, workspace_bytes,
+                           "av_degrid_double");
+  if (rc) return rc;
+  const int64_t rows = nt * nb * nvchan;
+  if (rows == 0 || nvpol == 0 || g_nchan == 0) return AV_OK;
+  cudaStream_t st = as_stream(stream);
+  rc = plan_build(g, p, uvw, freq, chanmap, 0.0, 0.0, st);
+  if (rc) return rc;
+  a.recs = p.recs;
+  a.tile_start = p.tile_start;
+  a.n_rec = p.offs + g.n_keys();
+  a.n_tiles = g.n_tiles();
+  a.ntu = g.ntu;
+  a.ntv = g.ntv;
+  a.cf_len = sampling * (support / 2 + 1);
+  switch (support) {
+    case 3: return launch_degrid_sorted<3>(a, rows, st);
+    case 4: return launch_degrid_sorted<4>(a, rows, st);
+    case 5: return launch_degrid_sorted<5>(a, rows, st);
+    case 6: return launch_degrid_sorted<6>(a, rows, st);
+    case 7: return launch_degrid_sorted<7>(a, rows, st);
+    case 8: return launch_degrid_sorted<8>(a, rows, st);
+    default: return launch_degrid_sorted<9>(a, rows, st);
+  }
 }
 
 }  // extern "C"

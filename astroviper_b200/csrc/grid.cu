@@ -167,8 +167,10 @@ struct TiledGridArgs {
   int a16;                 // vis and weight rows are 16-byte aligned (16-byte loads / copies)
   int64_t n_tiles, ntu, ntv;
   int64_t chunk;
-  const float2 *vis;
-  const float *wt;
+  const float2 *vis;       // complex64 data (NULL when vis64 holds complex128)
+  const float *wt;         // float32 weights (NULL when wt64 holds float64)
+  const double2 *vis64;    // double-precision inputs (SRC_F64)
+  const double *wt64;
   int do_psf;
   const double *cgk;
   int cgk_len, os;
@@ -187,6 +189,11 @@ struct TiledGridArgs {
   unsigned long long *det_sumw;  // (plane, npg)
   const double *det_scale;
 };
+
+// What the samples' values come from: complex64 data and float32 weights;
+// either or both in double precision; the degridder's adjoint (complex64
+// values with flags, scaled by 1 / sum of taps, no weights).
+enum GridSrc { SRC_F32, SRC_F64, SRC_ADJOINT };
 
 // Lane mappings.  Each warp streams its own contiguous slice of a tile
 // segment's cell-sorted samples, a whole run of samples in one cell (median
@@ -280,11 +287,15 @@ struct GCfg {
 // entry 0 for NPOL 1) and are replaced by the FP64 weighted values.  Entry
 // GT_STAGE of each plane (and of the offsets) is a zero sample that empty
 // group slots read.
-template <int S, int NPOL>
+// SRC_F64 and SRC_ADJOINT keep the next round's raw values in registers (a
+// double-precision sample of 4 polarisations has 96 raw bytes and 64 staged
+// ones) and one slot per warp; 24 more registers for SRC_F64 with NPOL 4 leave
+// room for 12 warps.
+template <int S, int NPOL, GridSrc SRC = SRC_F32>
 struct MCfg {
-  static constexpr int THREADS = 512;
+  static constexpr int THREADS = (SRC == SRC_F64 && NPOL == 4) ? 384 : 512;
   static constexpr int WARPS = THREADS / 32;
-  static constexpr int SLOTS = 2;                                  // rounds per ring
+  static constexpr int SLOTS = SRC == SRC_F32 ? 2 : 1;             // rounds per ring
   static constexpr int W = TILE + S - 1;
   static constexpr int RWP = 10;
   static constexpr int SDS = GT_STAGE + 1;
@@ -373,6 +384,69 @@ __device__ __forceinline__ void prefetch(Pref<NPOL> &f, const TiledGridArgs &a, 
       f.w[p] = p < a.npol ? __ldg(a.wt + vb + p) : 0.f;
       if (!a.do_psf) f.v[p] = p < a.npol ? __ldg(a.vis + vb + p) : make_float2(0.f, 0.f);
     }
+  }
+}
+
+// The same in double precision: each of the data and the weights may come in
+// either type.
+template <int NPOL>
+struct Pref64 {
+  Rec rc;
+  double w[NPOL];
+  double2 v[NPOL];
+  bool ok;
+};
+
+template <int NPOL>
+__device__ __forceinline__ void prefetch(Pref64<NPOL> &f, const TiledGridArgs &a, const Rec &rc,
+                                         bool valid) {
+  f.ok = valid;
+  if (!valid) return;
+  f.rc = rc;
+  const int64_t vb = (int64_t)rc.row * a.npol;
+#pragma unroll
+  for (int p = 0; p < NPOL; ++p) {
+    f.w[p] = 0.0;
+    f.v[p] = make_double2(0.0, 0.0);
+    if (p >= a.npol) continue;
+    f.w[p] = a.wt64 ? __ldg(a.wt64 + vb + p) : (double)__ldg(a.wt + vb + p);
+    if (a.do_psf) continue;
+    if (a.vis64) {
+      f.v[p] = __ldg(a.vis64 + vb + p);
+    } else {
+      const float2 x = __ldg(a.vis + vb + p);
+      f.v[p] = make_double2((double)x.x, (double)x.y);
+    }
+  }
+}
+
+template <int NPOL, GridSrc SRC>
+struct PrefOf {
+  using type = Pref<NPOL>;
+};
+template <int NPOL>
+struct PrefOf<NPOL, SRC_F64> {
+  using type = Pref64<NPOL>;
+};
+
+// FP64 weighted values of a prefetched sample, one plane of `stride` entries
+// per polarisation, and its share of the sums of weights (nrm: the sum of its
+// taps).  The reference skips NaN and exact-zero weighted data
+// (standard_grid.py:378).
+template <int NPOL, typename F>
+__device__ __forceinline__ void stage_values(const TiledGridArgs &a, const F &f, double nrm,
+                                             double2 *out, int stride, double (&sw)[NPOL]) {
+  double scl = 1.0;
+  if (a.inv_norm) scl = nrm != 0.0 ? 1.0 / nrm : 0.0;
+#pragma unroll
+  for (int p = 0; p < NPOL; ++p) {
+    double2 d;
+    if (a.do_psf) d = make_double2((double)f.w[p], 0.0);
+    else d = make_double2((double)f.v[p].x * (double)f.w[p] * scl,
+                          (double)f.v[p].y * (double)f.w[p] * scl);
+    const bool ok = p < a.npol && !isnan(d.x) && !isnan(d.y) && (d.x != 0.0 || d.y != 0.0);
+    out[p * stride] = ok ? d : make_double2(0.0, 0.0);
+    if (ok) sw[p] += (double)f.w[p] * nrm;
   }
 }
 
@@ -486,7 +560,7 @@ __device__ __forceinline__ void mma_f64_m16n8k4(double (&d)[4], double a0, doubl
 
 template <int S, int NPOL>
 struct MmaLanes {
-  using C = MCfg<S, NPOL>;
+  using C = MCfg<S, NPOL>;  // the strides do not depend on the source
   double acc[NPOL][4];  // per polarisation: re (g, 2t), re (g, 2t+1), im (g, 2t), im (g, 2t+1)
   int g, t;
   int ipm[NPOL];
@@ -674,7 +748,7 @@ __device__ __forceinline__ void rearm_schedule(const TiledGridArgs &a) {
 // Persistent: one CTA per SM takes chunks of records from a.sched[0] until
 // none are left; the last CTA to finish sets both counters back to zero for
 // the next launch on the same plan.
-template <int S, int NPOL>
+template <int S, int NPOL, GridSrc SRC>
 __global__ void __launch_bounds__(GCfg<S, NPOL>::THREADS, 1) k_grid_tiled(TiledGridArgs a) {
   using C = GCfg<S, NPOL>;
   constexpr int W = C::W, RWP = C::RWP;
@@ -745,13 +819,13 @@ __global__ void __launch_bounds__(GCfg<S, NPOL>::THREADS, 1) k_grid_tiled(TiledG
 
       // software pipeline: values of round rd + 1 and the record of round
       // rd + 2 are in flight while round rd is computed
-      Pref<NPOL> pf;
+      typename PrefOf<NPOL, SRC>::type pf;
       Rec rnext;
       {
         const uint32_t r = w_lo + lane;
         Rec r0;
         if (r < w_hi) r0 = a.recs[r];
-        prefetch<NPOL>(pf, a, r0, r < w_hi);
+        prefetch(pf, a, r0, r < w_hi);
       }
       bool rnext_ok = w_lo + GT_STAGE + lane < w_hi;
       if (rnext_ok) rnext = a.recs[w_lo + GT_STAGE + lane];
@@ -761,22 +835,7 @@ __global__ void __launch_bounds__(GCfg<S, NPOL>::THREADS, 1) k_grid_tiled(TiledG
         int my_key = -1;
         if (pf.ok) {
           const Rec rc = pf.rc;
-          const double nrm = rs[rc.ou] * rs[rc.ov];
-          double scl = 1.0;
-          if (a.inv_norm) scl = nrm != 0.0 ? 1.0 / nrm : 0.0;
-#pragma unroll
-          for (int p = 0; p < NPOL; ++p) {
-            double2 d;
-            if (a.do_psf) d = make_double2((double)pf.w[p], 0.0);
-            else d = make_double2((double)pf.v[p].x * (double)pf.w[p] * scl,
-                                  (double)pf.v[p].y * (double)pf.w[p] * scl);
-            // the reference skips NaN and exact-zero weighted data
-            // (standard_grid.py:378)
-            const bool ok = p < a.npol && !isnan(d.x) && !isnan(d.y) &&
-                            (d.x != 0.0 || d.y != 0.0);
-            wd[p * C::SDS + lane] = ok ? d : make_double2(0.0, 0.0);
-            if (ok) sw[p] += (double)pf.w[p] * nrm;
-          }
+          stage_values<NPOL>(a, pf, rs[rc.ou] * rs[rc.ov], wd + lane, C::SDS, sw);
           my_key = (int)rc.du | ((int)rc.dv << 8);
           wm[lane] = (int)rc.ou * RWP | (((int)rc.ov * RWP) << 16);
         }
@@ -788,7 +847,7 @@ __global__ void __launch_bounds__(GCfg<S, NPOL>::THREADS, 1) k_grid_tiled(TiledG
         __syncwarp();
         // ---- next round's values go out before this round is computed
         if (rd + 1 < n_rounds) {
-          prefetch<NPOL>(pf, a, rnext, rnext_ok);
+          prefetch(pf, a, rnext, rnext_ok);
           const uint32_t r = w_lo + (uint32_t)(rd + 2) * GT_STAGE + lane;
           rnext_ok = r < w_hi;
           if (rnext_ok) rnext = a.recs[r];
@@ -923,11 +982,12 @@ __device__ __forceinline__ void read_raw(const TiledGridArgs &a, const double2 *
 // two slots: the raw values of round rd + 1 are copied while round rd is
 // computed (a round of 32 samples takes several microseconds, well beyond
 // the copies' latency; a third slot, two rounds ahead, measured 3 % slower),
-// and records are loaded one round before their copies are issued.  Only
-// for weighted gridding (a.wt != NULL, no 1 / norm scaling).
-template <int S, int NPOL, bool DET = false>
-__global__ void __launch_bounds__(MCfg<S, NPOL>::THREADS, 1) k_grid_mma(TiledGridArgs a) {
-  using C = MCfg<S, NPOL>;
+// and records are loaded one round before their copies are issued.  The
+// other sources' raw values wait in registers instead of the ring.
+template <int S, int NPOL, bool DET = false, GridSrc SRC = SRC_F32>
+__global__ void __launch_bounds__(MCfg<S, NPOL, SRC>::THREADS, 1) k_grid_mma(TiledGridArgs a) {
+  using C = MCfg<S, NPOL, SRC>;
+  constexpr bool RING = SRC == SRC_F32;
   const double dscale = DET ? a.det_scale[0] : 0.0;
   const double wscale = DET ? a.det_scale[1] : 0.0;
   constexpr int W = C::W, RWP = C::RWP;
@@ -1010,15 +1070,25 @@ __global__ void __launch_bounds__(MCfg<S, NPOL>::THREADS, 1) k_grid_mma(TiledGri
       };
       rc0 = load_rec(0);
       rc1 = load_rec(1);
-      if (rc0.row != 0xffffffffu) issue_raw<NPOL>(a, wring, lane, rc0.row);
-      cp_async_commit();
+      typename PrefOf<NPOL, SRC>::type pf;
+      if constexpr (RING) {
+        if (rc0.row != 0xffffffffu) issue_raw<NPOL>(a, wring, lane, rc0.row);
+        cp_async_commit();
+      } else {
+        prefetch(pf, a, rc0, rc0.row != 0xffffffffu);
+      }
       for (int rd = 0; rd < n_rounds; ++rd) {
         double2 *slot = wring + (rd % C::SLOTS) * C::SLOT;
-        cp_async_wait<0>();  // this lane's copies of round rd are complete
+        if (RING) cp_async_wait<0>();  // this lane's copies of round rd are complete
         // ---- stage: FP64 weighted values in place of the raw ones, the
         // cell key and the offsets of the two tap-table rows
         int my_key = -1;
-        if (rc0.row != 0xffffffffu) {
+        if (!RING && rc0.row != 0xffffffffu) {
+          stage_values<NPOL>(a, pf, rs[rc0.ou] * rs[rc0.ov], slot + lane, C::SDS, sw);
+          my_key = (int)rc0.du | ((int)rc0.dv << 8);
+          wm[lane] = (int)rc0.ou * RWP | (((int)rc0.ov * RWP) << 16);
+        }
+        if (RING && rc0.row != 0xffffffffu) {
           float2 v[NPOL];
           float w[NPOL];
           read_raw<NPOL>(a, slot, lane, v, w);
@@ -1052,9 +1122,13 @@ __global__ void __launch_bounds__(MCfg<S, NPOL>::THREADS, 1) k_grid_mma(TiledGri
         const unsigned starts = __ballot_sync(0xffffffffu, my_key >= 0 && my_key != prev);
         // ---- copies of round rd + 1 (into the slot round rd - 1 used) and
         // the record of round rd + 2
-        if (rc1.row != 0xffffffffu)
-          issue_raw<NPOL>(a, wring + ((rd + 1) % C::SLOTS) * C::SLOT, lane, rc1.row);
-        cp_async_commit();
+        if constexpr (RING) {
+          if (rc1.row != 0xffffffffu)
+            issue_raw<NPOL>(a, wring + ((rd + 1) % C::SLOTS) * C::SLOT, lane, rc1.row);
+          cp_async_commit();
+        } else {
+          prefetch(pf, a, rc1, rc1.row != 0xffffffffu);
+        }
         const Rec rc2 = load_rec(rd + 2);
         __syncwarp();
         // ---- compute the round's samples in runs of one cell
@@ -1082,7 +1156,7 @@ __global__ void __launch_bounds__(MCfg<S, NPOL>::THREADS, 1) k_grid_mma(TiledGri
         rc0 = rc1;
         rc1 = rc2;
       }
-      cp_async_wait<0>();
+      if (RING) cp_async_wait<0>();
       if (cur >= 0) lanes.template flush<DET>(sre, sim, cur, dscale);
       if (DET) add_sum_weight_det<NPOL>(a, sw, pm, plane, lane, wscale);
       else add_sum_weight<NPOL>(a, sw, pm, plane, lane);
@@ -1097,7 +1171,7 @@ __global__ void __launch_bounds__(MCfg<S, NPOL>::THREADS, 1) k_grid_mma(TiledGri
   rearm_schedule(a);
 }
 
-template <int S, int NPOL>
+template <int S, int NPOL, GridSrc SRC>
 static int launch_grid_rows(const TiledGridArgs &a, int64_t nblocks, cudaStream_t st) {
   using C = GCfg<S, NPOL>;
   size_t smem = C::total(a.npg);
@@ -1105,44 +1179,54 @@ static int launch_grid_rows(const TiledGridArgs &a, int64_t nblocks, cudaStream_
   int dev = 0;
   AV_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    AV_CUDA(cudaFuncSetAttribute(k_grid_tiled<S, NPOL>,
+    AV_CUDA(cudaFuncSetAttribute(k_grid_tiled<S, NPOL, SRC>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::total(4)));
     configured[dev] = true;
   }
-  k_grid_tiled<S, NPOL><<<(unsigned)nblocks, C::THREADS, smem, st>>>(a);
+  k_grid_tiled<S, NPOL, SRC><<<(unsigned)nblocks, C::THREADS, smem, st>>>(a);
   AV_LAUNCH_CHECK();
   return AV_OK;
 }
 
-template <int S, int NPOL, bool DET = false>
+template <int S, int NPOL, bool DET = false, GridSrc SRC = SRC_F32>
 static int launch_grid_mma(const TiledGridArgs &a, int64_t nblocks, cudaStream_t st) {
-  using C = MCfg<S, NPOL>;
+  using C = MCfg<S, NPOL, SRC>;
   size_t smem = C::total(a.npg);
   static bool configured[64] = {false};
   int dev = 0;
   AV_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    AV_CUDA(cudaFuncSetAttribute(k_grid_mma<S, NPOL, DET>,
+    AV_CUDA(cudaFuncSetAttribute(k_grid_mma<S, NPOL, DET, SRC>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::total(4)));
     configured[dev] = true;
   }
-  k_grid_mma<S, NPOL, DET><<<(unsigned)nblocks, C::THREADS, smem, st>>>(a);
+  k_grid_mma<S, NPOL, DET, SRC><<<(unsigned)nblocks, C::THREADS, smem, st>>>(a);
   AV_LAUNCH_CHECK();
   return AV_OK;
 }
 
-// k_grid_mma for weighted gridding as the AV_TUNE_GRID_LANES knob says
-// (automatically for supports 5-8: with smaller footprints most of the 8 x 8
-// tile is padding and the row lanes are faster); k_grid_tiled otherwise
-// (support 9, the degridder's adjoint).
+// k_grid_mma as the AV_TUNE_GRID_LANES knob says (automatically for supports
+// 5-8: with smaller footprints most of the 8 x 8 tile is padding and the row
+// lanes are faster); k_grid_tiled otherwise (support 9).  The degridder's
+// adjoint follows the same rule: 4.16M samples of one polarisation, support 7,
+// take 145 us against 210 us of the row lanes.  Double-precision inputs take
+// k_grid_mma for every support it covers, whatever the knob says: 806k
+// samples of 2 polarisations take 78 us, and 31 us of plan, against 2620 us of
+// k_grid_plain, whose 98 global FP64 atomics per correlation bound it.
 template <int S, int NPOL>
 static int launch_grid_tiled(const TiledGridArgs &a, int64_t nblocks, cudaStream_t st) {
+  const bool f64 = a.wt64 != nullptr || a.vis64 != nullptr;
   if constexpr (S <= 8) {
+    if (f64) return launch_grid_mma<S, NPOL, false, SRC_F64>(a, nblocks, st);
     const int64_t lanes = tune_value(AV_TUNE_GRID_LANES);
-    const bool mma = lanes == AV_GRID_LANES_MMA || (lanes == AV_GRID_LANES_AUTO && S >= 5);
-    if (a.wt != nullptr && !a.inv_norm && mma) return launch_grid_mma<S, NPOL>(a, nblocks, st);
+    if (lanes == AV_GRID_LANES_MMA || (lanes == AV_GRID_LANES_AUTO && S >= 5)) {
+      if (a.wt == nullptr) return launch_grid_mma<S, NPOL, false, SRC_ADJOINT>(a, nblocks, st);
+      return launch_grid_mma<S, NPOL>(a, nblocks, st);
+    }
+  } else {
+    if (f64) return launch_grid_rows<S, NPOL, SRC_F64>(a, nblocks, st);
   }
-  return launch_grid_rows<S, NPOL>(a, nblocks, st);
+  return launch_grid_rows<S, NPOL, SRC_F32>(a, nblocks, st);
 }
 
 template <int S>
@@ -1462,26 +1546,17 @@ int av_tiled_plan_counts(int64_t nt, int64_t nb, int64_t nchan, int64_t n_u, int
   return AV_OK;
 }
 
-int av_grid_tiled_execute(void *grid, int grid_dtype, double *sum_weight, int do_psf,
-                          const void *vis, int vis_dtype, const void *weight, int weight_dtype,
-                          const int32_t *pol_map, const double *cgk, int64_t n_u, int64_t n_v,
-                          int support, int oversampling, int64_t nt, int64_t nb, int64_t nchan,
-                          int64_t npol, int64_t n_img_chan, int64_t n_img_pol, void *workspace,
-                          size_t workspace_bytes, void *stream) {
-  clear_error();
-  AV_CHECK_ARG(grid && sum_weight && weight && pol_map && cgk,
-               "av_grid_tiled_execute: null pointer");
-  AV_CHECK_ARG(do_psf || vis, "av_grid_tiled_execute: vis is required unless do_psf");
-  AV_CHECK_ARG(grid_dtype == AV_C64 || grid_dtype == AV_C128,
-               "av_grid_tiled_execute: grid must be complex64 or complex128");
-  AV_CHECK_ARG(do_psf || vis_dtype == AV_C64, "av_grid_tiled_execute: vis must be complex64");
-  AV_CHECK_ARG(weight_dtype == AV_F32, "av_grid_tiled_execute: weight must be float32");
-  AV_CHECK_ARG(npol >= 0 && npol <= 4 && n_img_pol >= 1 && n_img_pol <= 4,
-               "av_grid_tiled_execute: npol and n_img_pol must be in [1, 4]");
+// The execute half on inputs of any of the types (checked by the callers).
+static int grid_execute(const char *who, void *grid, int grid_dtype, double *sum_weight,
+                        int do_psf, const void *vis, int vis_dtype, const void *weight,
+                        int weight_dtype, const int32_t *pol_map, const double *cgk, int64_t n_u,
+                        int64_t n_v, int support, int oversampling, int64_t nt, int64_t nb,
+                        int64_t nchan, int64_t npol, int64_t n_img_chan, int64_t n_img_pol,
+                        void *workspace, size_t workspace_bytes, void *stream) {
   PlanGeom g;
   Plan p;
   int rc = grid_geom_checked(g, n_u, n_v, support, oversampling, nt, nb, nchan, n_img_chan,
-                             workspace, workspace_bytes, p, "av_grid_tiled_execute");
+                             workspace, workspace_bytes, p, who);
   if (rc) return rc;
   int64_t rows = nt * nb * nchan;
   if (rows == 0 || npol == 0) return AV_OK;
@@ -1496,8 +1571,11 @@ int av_grid_tiled_execute(void *grid, int grid_dtype, double *sum_weight, int do
   int64_t nblocks = 0;
   a.chunk = grid_chunking(rows, nblocks);
   a.sched = p.counters;
-  a.vis = (const float2 *)vis;
-  a.wt = (const float *)weight;
+  const bool v64 = !do_psf && vis_dtype == AV_C128, w64 = weight_dtype == AV_F64;
+  a.vis = v64 ? nullptr : (const float2 *)vis;
+  a.wt = w64 ? nullptr : (const float *)weight;
+  a.vis64 = v64 ? (const double2 *)vis : nullptr;
+  a.wt64 = w64 ? (const double *)weight : nullptr;
   a.do_psf = do_psf;
   a.cgk = cgk;
   a.cgk_len = oversampling * (support / 2 + 1);
@@ -1518,6 +1596,28 @@ int av_grid_tiled_execute(void *grid, int grid_dtype, double *sum_weight, int do
     a.a16 = v16 && ((npol == 4 && wp % 16 == 0) || (npol == 2 && wp % 8 == 0));
   }
   return dispatch_support(a, support, npol_t, nblocks, as_stream(stream));
+}
+
+int av_grid_tiled_execute(void *grid, int grid_dtype, double *sum_weight, int do_psf,
+                          const void *vis, int vis_dtype, const void *weight, int weight_dtype,
+                          const int32_t *pol_map, const double *cgk, int64_t n_u, int64_t n_v,
+                          int support, int oversampling, int64_t nt, int64_t nb, int64_t nchan,
+                          int64_t npol, int64_t n_img_chan, int64_t n_img_pol, void *workspace,
+                          size_t workspace_bytes, void *stream) {
+  clear_error();
+  AV_CHECK_ARG(grid && sum_weight && weight && pol_map && cgk,
+               "av_grid_tiled_execute: null pointer");
+  AV_CHECK_ARG(do_psf || vis, "av_grid_tiled_execute: vis is required unless do_psf");
+  AV_CHECK_ARG(grid_dtype == AV_C64 || grid_dtype == AV_C128,
+               "av_grid_tiled_execute: grid must be complex64 or complex128");
+  AV_CHECK_ARG(do_psf || vis_dtype == AV_C64, "av_grid_tiled_execute: vis must be complex64");
+  AV_CHECK_ARG(weight_dtype == AV_F32, "av_grid_tiled_execute: weight must be float32");
+  AV_CHECK_ARG(npol >= 0 && npol <= 4 && n_img_pol >= 1 && n_img_pol <= 4,
+               "av_grid_tiled_execute: npol and n_img_pol must be in [1, 4]");
+  return grid_execute("av_grid_tiled_execute", grid, grid_dtype, sum_weight, do_psf, vis,
+                      vis_dtype, weight, weight_dtype, pol_map, cgk, n_u, n_v, support,
+                      oversampling, nt, nb, nchan, npol, n_img_chan, n_img_pol, workspace,
+                      workspace_bytes, stream);
 }
 
 int av_tiled_plan_order_rows(int64_t nt, int64_t nb, int64_t nchan, int64_t n_u, int64_t n_v,
@@ -1600,6 +1700,8 @@ int av_grid_tiled_execute_det(void *grid, int grid_dtype, double *sum_weight, in
   a.sched = p.counters;
   a.vis = (const float2 *)vis;
   a.wt = (const float *)weight;
+  a.vis64 = nullptr;
+  a.wt64 = nullptr;
   a.do_psf = do_psf;
   a.cgk = cgk;
   a.cgk_len = oversampling * (support / 2 + 1);
@@ -1705,6 +1807,8 @@ int av_degrid_tiled_adjoint(void *grid, int grid_dtype, const void *values, int 
   a.sched = p.counters;
   a.vis = (const float2 *)values;
   a.wt = nullptr;
+  a.vis64 = nullptr;
+  a.wt64 = nullptr;
   a.do_psf = 0;
   a.cgk = convFunc;
   a.cgk_len = sampling * (support / 2 + 1);
@@ -1739,6 +1843,34 @@ int av_grid_tiled(void *grid, int grid_dtype, double *sum_weight, int do_psf,
                                weight_dtype, pol_map, cgk, n_u, n_v, support, oversampling, nt,
                                nb, nchan, npol, n_img_chan, n_img_pol, workspace,
                                workspace_bytes, stream);
+}
+
+int av_grid_double(void *grid, int grid_dtype, double *sum_weight, int do_psf, const void *vis,
+                   int vis_dtype, const void *weight, int weight_dtype, const double *uvw,
+                   const double *freq, const int32_t *chan_map, const int32_t *pol_map,
+                   const double *cgk, int64_t n_u, int64_t n_v, double delta_l, double delta_m,
+                   int support, int oversampling, int64_t nt, int64_t nb, int64_t nchan,
+                   int64_t npol, int64_t n_img_chan, int64_t n_img_pol, void *workspace,
+                   size_t workspace_bytes, void *stream) {
+  clear_error();
+  AV_CHECK_ARG(grid && sum_weight && weight && uvw && freq && chan_map && pol_map && cgk,
+               "av_grid_double: null pointer");
+  AV_CHECK_ARG(do_psf || vis, "av_grid_double: vis is required unless do_psf");
+  AV_CHECK_ARG(grid_dtype == AV_C64 || grid_dtype == AV_C128,
+               "av_grid_double: grid must be complex64 or complex128");
+  AV_CHECK_ARG(do_psf || vis_dtype == AV_C64 || vis_dtype == AV_C128,
+               "av_grid_double: vis must be complex64 or complex128");
+  AV_CHECK_ARG(weight_dtype == AV_F32 || weight_dtype == AV_F64,
+               "av_grid_double: weight must be float32 or float64");
+  AV_CHECK_ARG(npol >= 0 && npol <= 4 && n_img_pol >= 1 && n_img_pol <= 4,
+               "av_grid_double: npol and n_img_pol must be in [1, 4]");
+  int rc = av_grid_tiled_plan(uvw, freq, chan_map, n_u, n_v, delta_l, delta_m, support,
+                              oversampling, nt, nb, nchan, n_img_chan, workspace,
+                              workspace_bytes, stream);
+  if (rc) return rc;
+  return grid_execute("av_grid_double", grid, grid_dtype, sum_weight, do_psf, vis, vis_dtype,
+                      weight, weight_dtype, pol_map, cgk, n_u, n_v, support, oversampling, nt, nb,
+                      nchan, npol, n_img_chan, n_img_pol, workspace, workspace_bytes, stream);
 }
 
 }  // extern "C"

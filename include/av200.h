@@ -202,6 +202,18 @@ int av_grid_tiled(void *grid, int grid_dtype, double *sum_weight, int do_psf,
                   int64_t nb, int64_t nchan, int64_t npol, int64_t n_img_chan,
                   int64_t n_img_pol, void *workspace, size_t workspace_bytes, void *stream);
 
+/* av_grid_tiled with complex64 or complex128 visibilities and float32 or
+ * float64 weights, products and sums in FP64: av_grid_plain's results to
+ * within summation order, for the shapes that av_grid_tiled covers (same
+ * workspace). */
+int av_grid_double(void *grid, int grid_dtype, double *sum_weight, int do_psf, const void *vis,
+                   int vis_dtype, const void *weight, int weight_dtype, const double *uvw,
+                   const double *freq, const int32_t *chan_map, const int32_t *pol_map,
+                   const double *cgk, int64_t n_u, int64_t n_v, double delta_l, double delta_m,
+                   int support, int oversampling, int64_t nt, int64_t nb, int64_t nchan,
+                   int64_t npol, int64_t n_img_chan, int64_t n_img_pol, void *workspace,
+                   size_t workspace_bytes, void *stream);
+
 /* No counterpart in the reference: av_grid_tiled_plan that also leaves out
  * the samples whose every weight is zero or NaN (flagged data), which
  * standard_grid_jit skips (standard_grid.py:378), so that grids with many
@@ -314,6 +326,17 @@ int av_degrid_plain_adjoint(const double *uvw, const double *dphase, const void 
                             const double *convFunc, const int32_t *chanmap,
                             const int32_t *polmap, int64_t nt, int64_t nb, int64_t nvchan,
                             int64_t nvpol, void *stream);
+
+/* av_degrid_plain (values +=, bit-identical) with the samples binned by cell
+ * first, for 3 <= support <= 9, sampling <= 254, nvpol <= 4 and c =
+ * 299792458; workspace of av_degrid_tiled_workspace_size. */
+int av_degrid_double(const double *uvw, const double *dphase, void *values, int values_dtype,
+                     const uint8_t *flag, double scale_x, double scale_y, double offset_x,
+                     double offset_y, const void *grid, int grid_dtype, int64_t g_nchan,
+                     int64_t g_npol, int64_t g_n2, int64_t g_n3, const double *freq, int support,
+                     int sampling, const double *convFunc, const int32_t *chanmap,
+                     const int32_t *polmap, int64_t nt, int64_t nb, int64_t nvchan,
+                     int64_t nvpol, void *workspace, size_t workspace_bytes, void *stream);
 
 size_t av_degrid_tiled_workspace_size(int64_t nt, int64_t nb, int64_t nvchan, int64_t g_n2,
                                       int64_t g_n3, int64_t g_nchan, int support);
