@@ -784,6 +784,17 @@ def mosaic_grid(grid, sum_weight, do_psf, vis, weight, uvw, freq, chan_map, pol_
                                      float(delta_lm[0]), float(delta_lm[1]), max_sup, os_u, nt,
                                      nb, nchan, n_img_chan, wptr, wbytes, stream_ptr()),
           "av_mosaic_tiled_plan")
+    # the kernel with the footprint in registers, unless gathering the taps of
+    # every kernel offset would be more work than reading the functions a few
+    # times (windows much wider than the support), or has no room
+    n_cf = n_cfb * n_cfc * n_cfp
+    taps = n_cf * (os_u + 1) ** 2 * max_sup ** 2
+    if max_sup <= 11 and npol <= 4 and taps <= 4 * n_cf * cu * cv + (1 << 20):
+        tab = _scratch(lib().av_mosaic_taps_size(n_cf, max_sup, os_u))
+        if tab is not None:
+            check(lib().av_mosaic_runs_execute(*args, wptr, wbytes, tab[1], tab[2],
+                                               stream_ptr()), "av_mosaic_runs_execute")
+            return grid, sum_weight
     check(lib().av_mosaic_tiled_execute(*args, wptr, wbytes, stream_ptr()),
           "av_mosaic_tiled_execute")
     return grid, sum_weight

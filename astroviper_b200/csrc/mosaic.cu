@@ -14,6 +14,8 @@
 //                     its function once.
 // av_cf_phase_product conv_kernel x phase_gradient[0] (mosaic_grid.py:384,
 //                     :56-58), elementwise without fused multiply-add.
+#include <algorithm>
+
 #include "plan.cuh"
 
 namespace av {
@@ -484,6 +486,407 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mosaic_tiled(MosaicTiledArgs 
   }
 }
 
+// ------------------------------------------------------------------ runs --
+// The same binned gridding for windows of up to MR_MAX_S cells and up to 4
+// polarisations, with the footprint in registers: the kernel above spends
+// some 640 instructions on a sample (a whole warp per sample and
+// polarisation, the sample's indices worked out by every lane, two shared
+// FP64 atomics per tap).  Here
+//   - the taps of every function and kernel offset are first gathered into
+//     contiguous rows of S x S values (k_mosaic_taps), with the row's norm, so
+//     a sample's taps are one coalesced read where the oversampled function
+//     spreads them over a 32-byte sector each;
+//   - a warp's lanes stage 32 samples at once (weighted values, tap row, sum
+//     of weights), the next round's data in flight meanwhile;
+//   - lane l owns window cells l, l + 32, ... and keeps their sums for all
+//     polarisations while the samples stay in one cell: one tap load and 4
+//     NPOL DFMA per sample and owned cell, shared atomics only when the cell
+//     changes; four samples' taps are in flight whatever the runs.
+// Cells past the window hold zero taps, so only an infinite value, whose
+// product with them would be NaN, needs the window's true extent; such
+// samples (rare) are masked tap by tap.
+// 1.03M samples x 2 polarisations, supports 5-7: 1315 us before, 257 us now (and 70 us of plan).
+constexpr int MR_MAX_S = 11;
+constexpr int MR_THREADS = 256;
+constexpr int MR_WARPS = MR_THREADS / 32;
+constexpr int MR_ROUND = 32;  // samples a warp stages at once
+
+struct MosaicRunsArgs {
+  MosaicTiledArgs t;
+  const double2 *taps;  // [function][u offset][v offset][S * S]
+  const double *norm;   // Re(norm) (PSF) or Re(norm^2) of each row
+  int first, n_off;     // kernel offsets first .. first + n_off - 1
+};
+
+// Whether tap (iu, iv) counted from the window's corner is one of function
+// fidx's at offset (ou, ov), and where it is.
+__device__ __forceinline__ bool mosaic_tap(const MosaicArgs &a, int64_t fidx, int S, int ri,
+                                           int ci, int ou, int ov, int64_t &at) {
+  const int su = a.support[2 * fidx], sv = a.support[2 * fidx + 1];
+  const int iu = ri - S / 2, iv = ci - S / 2;
+  const int64_t fu = (int64_t)a.os_u * iu + ou + a.cu / 2;
+  const int64_t fv = (int64_t)a.os_v * iv + ov + a.cv / 2;
+  at = fidx * a.cu * a.cv + fu * a.cv + fv;
+  return su >= 1 && sv >= 1 && su <= S && sv <= S && iu >= -(su / 2) && iu < su - su / 2 &&
+         iv >= -(sv / 2) && iv < sv - sv / 2 && fu >= 0 && fu < a.cu && fv >= 0 && fv < a.cv;
+}
+
+// One block per (function, u offset, v offset).
+__global__ void __launch_bounds__(128) k_mosaic_taps(MosaicArgs a, int S, int first, int n_off,
+                                                     double2 *taps, double *norm) {
+  const int64_t row = blockIdx.x;
+  const int ov = first + (int)(row % n_off), ou = first + (int)(row / n_off % n_off);
+  const int64_t fidx = row / ((int64_t)n_off * n_off);
+  double2 c = make_double2(0.0, 0.0);
+  const int i = threadIdx.x;
+  if (i < S * S) {
+    int64_t at;
+    if (mosaic_tap(a, fidx, S, i / S, i % S, ou, ov, at)) c = a.cf[at];
+    taps[row * (S * S) + i] = c;
+  }
+  __shared__ double2 sh[4];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    c.x += __shfl_down_sync(0xffffffffu, c.x, o);
+    c.y += __shfl_down_sync(0xffffffffu, c.y, o);
+  }
+  if ((i & 31) == 0) sh[i >> 5] = c;
+  __syncthreads();
+  if (i == 0) {
+    const double x = (sh[0].x + sh[1].x) + (sh[2].x + sh[3].x);
+    const double y = (sh[0].y + sh[1].y) + (sh[2].y + sh[3].y);
+    norm[row] = a.do_psf ? x : __dsub_rn(__dmul_rn(x, x), __dmul_rn(y, y));
+  }
+}
+
+// A sample's record and raw values, in flight until used.
+template <int NPOL>
+struct MosaicRaw {
+  Rec rc;
+  bool ok;
+  double w[NPOL];
+  double2 v[NPOL];
+};
+
+template <int NPOL>
+__device__ __forceinline__ void mosaic_fetch(MosaicRaw<NPOL> &f, const MosaicArgs &a,
+                                             const Rec &rc, bool ok) {
+  f.ok = ok;
+  if (!ok) return;
+  f.rc = rc;
+  const int64_t k = (int64_t)rc.row * a.npol;
+#pragma unroll
+  for (int p = 0; p < NPOL; ++p) {
+    f.w[p] = p < a.npol ? __ldg(a.wt + k + p) : 0.0;
+    f.v[p] = p < a.npol && !a.do_psf ? __ldg(a.vis + k + p) : make_double2(0.0, 0.0);
+  }
+}
+
+struct MosaicShape {  // sub-grid strides: odd rows, planes 1 mod 16 doubles
+  int W, RS, PS;
+  __host__ __device__ explicit MosaicShape(int S)
+      : W(TILE + S - 1), RS(W | 1), PS((W * RS + 15) / 16 * 16 + 1) {}
+};
+
+template <int NPOL>
+__host__ __device__ constexpr size_t mosaic_stage_bytes() {
+  return (size_t)MR_WARPS * MR_ROUND * NPOL * (sizeof(double2) + sizeof(int));
+}
+
+// Round slots: value [pol][sample], tap row [pol][sample].
+template <int CPL, int NPOL, bool MULTI>
+struct MosaicLanes {
+  double2 acc[CPL][NPOL];
+  int cell[CPL];  // offset of the owned cells in the sub-grid
+  bool own[CPL];
+  int ipm[NPOL];
+
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int c = 0; c < CPL; ++c)
+#pragma unroll
+      for (int p = 0; p < NPOL; ++p) acc[c][p] = make_double2(0.0, 0.0);
+  }
+
+  __device__ __forceinline__ void add(int c, int p, double2 k, double2 d) {
+    double2 &x = acc[c][p];
+    x.x = fma(k.x, d.x, x.x);
+    x.y = fma(k.x, d.y, x.y);
+    x.x = fma(-k.y, d.y, x.x);
+    x.y = fma(k.y, d.x, x.y);
+  }
+
+  __device__ __forceinline__ void flush(double *sre, double *sim, int key,
+                                        const MosaicShape &m) {
+    const int base = (key & 255) * m.RS + ((key >> 8) & 255);
+#pragma unroll
+    for (int c = 0; c < CPL; ++c)
+#pragma unroll
+      for (int p = 0; p < NPOL; ++p) {
+        const double2 v = acc[c][p];
+        if (own[c] && ipm[p] >= 0 && (v.x != 0.0 || v.y != 0.0)) {
+          const int e = ipm[p] * m.PS + base + cell[c];
+          atomicAdd(sre + e, v.x);
+          atomicAdd(sim + e, v.y);
+        }
+      }
+    clear();
+  }
+};
+
+template <int CPL, int NPOL, bool MULTI>
+__global__ void __launch_bounds__(MR_THREADS, CPL *NPOL <= 4 ? 2 : 1)
+    k_mosaic_runs(MosaicRunsArgs q) {
+  const MosaicTiledArgs &t = q.t;
+  const MosaicArgs &a = t.m;
+  constexpr int NF = MULTI ? NPOL : 1;  // tap rows per sample
+  // samples whose taps are loaded together: up to 8 loads in flight per lane
+  constexpr int AHEAD = NF * CPL <= 2 ? 4 : (NF * CPL <= 4 ? 2 : 1);
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int S = t.S, S2 = S * S, npg = (int)a.n_img_pol;
+  const MosaicShape m(S);
+  double2 *wd = (double2 *)smem + warp * MR_ROUND * NPOL;
+  int *tr = (int *)(smem + (size_t)MR_WARPS * MR_ROUND * NPOL * sizeof(double2)) +
+            warp * MR_ROUND * NPOL;
+  double *sre = (double *)(smem + mosaic_stage_bytes<NPOL>());
+  double *sim = sre + (size_t)npg * m.PS;
+  __shared__ int s_chunk;
+
+  MosaicLanes<CPL, NPOL, MULTI> lanes;
+  int cfp[NPOL];
+#pragma unroll
+  for (int p = 0; p < NPOL; ++p) {
+    const int ap = p < a.npol ? a.pol_map[p] : -1;
+    cfp[p] = p < a.npol ? a.cfp_map[p] : -1;
+    lanes.ipm[p] = ap >= 0 && ap < npg && cfp[p] >= 0 && cfp[p] < a.n_cfp ? ap : -1;
+  }
+#pragma unroll
+  for (int c = 0; c < CPL; ++c) {
+    const int i = lane + 32 * c;
+    lanes.own[c] = i < S2;
+    lanes.cell[c] = (i / S) * m.RS + i % S;
+  }
+  lanes.clear();
+  for (int i0 = 0; i0 < 2 * npg * m.PS; i0 += MR_THREADS) {
+    const int i = i0 + threadIdx.x;
+    if (i < 2 * npg * m.PS) sre[i] = 0.0;
+  }
+  const uint32_t n_rec = *t.n_rec;
+  const int64_t n_chunks = ((int64_t)n_rec + t.chunk - 1) / t.chunk;
+  for (;;) {
+    __syncthreads();  // sub-grid clear; previous s_chunk consumed
+    if (threadIdx.x == 0) s_chunk = (int)atomicAdd(&t.sched[0], 1u);
+    __syncthreads();
+    const int64_t ch = s_chunk;
+    if (ch >= n_chunks) break;
+    const uint32_t r0 = (uint32_t)(ch * t.chunk);
+    const uint32_t r1 = (uint32_t)min((int64_t)n_rec, (int64_t)r0 + t.chunk);
+    int64_t tile = find_tile_warp(t.tile_start, t.n_tiles, r0);
+    uint32_t seg_lo = r0;
+    while (seg_lo < r1) {
+      const uint32_t t_end = t.tile_start[tile + 1];
+      const uint32_t seg_hi = min(r1, t_end);
+      if (seg_hi <= seg_lo) {
+        ++tile;
+        continue;
+      }
+      const int64_t plane = tile / (t.ntu * t.ntv);
+      const int64_t trem = tile - plane * t.ntu * t.ntv;
+      const int tu = (int)(trem / t.ntv), tv = (int)(trem - (int64_t)tu * t.ntv);
+      const uint32_t seg_n = seg_hi - seg_lo;
+      const uint32_t w_lo = seg_lo + (uint32_t)(((uint64_t)seg_n * warp) / MR_WARPS);
+      const uint32_t w_hi = seg_lo + (uint32_t)(((uint64_t)seg_n * (warp + 1)) / MR_WARPS);
+      const int n_rounds = (int)((w_hi - w_lo + MR_ROUND - 1) / MR_ROUND);
+      int cur = -1;
+      double sw[NPOL];
+#pragma unroll
+      for (int p = 0; p < NPOL; ++p) sw[p] = 0.0;
+      auto load_rec = [&](int rd) {
+        const uint32_t r = w_lo + (uint32_t)rd * MR_ROUND + lane;
+        Rec x;
+        if (rd < n_rounds && r < w_hi) x = t.recs[r];
+        else x.row = 0xffffffffu;
+        return x;
+      };
+      MosaicRaw<NPOL> raw;
+      Rec next = load_rec(0);
+      mosaic_fetch<NPOL>(raw, a, next, next.row != 0xffffffffu);
+      next = load_rec(1);
+      for (int rd = 0; rd < n_rounds; ++rd) {
+        // ---- stage one sample per lane
+        int key = -1;
+        bool inf = false;
+        if (raw.ok) {
+          const Rec rc = raw.rc;
+          const uint32_t tb = fdiv(rc.row, t.div_nchan);
+          const uint32_t c = rc.row - tb * (uint32_t)a.nchan;
+          const uint32_t b = tb - fdiv(tb, t.div_nb) * (uint32_t)a.nb;
+          const int cfb = a.cfb_map[b], cfc = a.cfc_map[c];
+          const bool has = cfb >= 0 && cfb < a.n_cfb && cfc >= 0 && cfc < a.n_cfc;
+          const int ou = min(max((int)rc.ou - 128 - q.first, 0), q.n_off - 1);
+          const int ov = min(max((int)rc.ov - 128 - q.first, 0), q.n_off - 1);
+          if (!MULTI) tr[lane] = 0;
+#pragma unroll
+          for (int p = 0; p < NPOL; ++p) {
+            double2 d;
+            if (a.do_psf) d = make_double2(raw.w[p], 0.0);
+            else d = make_double2(__dmul_rn(raw.v[p].x, raw.w[p]),
+                                  __dmul_rn(raw.v[p].y, raw.w[p]));
+            bool ok = has && lanes.ipm[p] >= 0 && !isnan(d.x) && !isnan(d.y) &&
+                      (d.x != 0.0 || d.y != 0.0);
+            int row = 0;
+            if (ok) {
+              const int64_t fidx = ((int64_t)cfb * a.n_cfc + cfc) * a.n_cfp + cfp[p];
+              const int su = a.support[2 * fidx], sv = a.support[2 * fidx + 1];
+              // a window larger than the plan's footprint (max_support) is skipped
+              ok = su >= 1 && sv >= 1 && su <= S && sv <= S;
+              row = (int)((fidx * q.n_off + ou) * q.n_off + ov);
+            }
+            wd[p * MR_ROUND + lane] = ok ? d : make_double2(0.0, 0.0);
+            if (ok) {
+              sw[p] += __dmul_rn(raw.w[p], __ldg(q.norm + row));
+              inf |= isinf(d.x) || isinf(d.y);
+            }
+            if (MULTI || ok) tr[(MULTI ? p : 0) * MR_ROUND + lane] = row;
+          }
+          key = (int)rc.du | ((int)rc.dv << 8);
+        }
+        int prev = __shfl_up_sync(0xffffffffu, key, 1);
+        if (lane == 0) prev = cur;
+        const unsigned starts = __ballot_sync(0xffffffffu, key >= 0 && key != prev);
+        const unsigned infs = __ballot_sync(0xffffffffu, inf);
+        // ---- the next round's loads, before this one is computed
+        mosaic_fetch<NPOL>(raw, a, next, next.row != 0xffffffffu);
+        next = load_rec(rd + 2);
+        __syncwarp();
+        const int jn = (int)min((uint32_t)MR_ROUND, w_hi - (w_lo + (uint32_t)rd * MR_ROUND));
+        if (infs == 0u) {
+          for (int j0 = 0; j0 < jn; j0 += AHEAD) {
+            double2 cv[AHEAD][NF][CPL];
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u)
+#pragma unroll
+              for (int f = 0; f < NF; ++f) {
+                const int j = min(j0 + u, jn - 1);
+                const double2 *row = q.taps + (int64_t)tr[f * MR_ROUND + j] * S2;
+#pragma unroll
+                for (int c = 0; c < CPL; ++c)
+                  cv[u][f][c] =
+                      lanes.own[c] ? __ldg(row + lane + 32 * c) : make_double2(0.0, 0.0);
+              }
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+              const int j = j0 + u;
+              if (j >= jn) break;
+              if ((starts >> j) & 1u) {
+                if (cur >= 0) lanes.flush(sre, sim, cur, m);
+                cur = __shfl_sync(0xffffffffu, key, j);
+              }
+#pragma unroll
+              for (int p = 0; p < NPOL; ++p)
+#pragma unroll
+                for (int c = 0; c < CPL; ++c)
+                  lanes.add(c, p, cv[u][MULTI ? p : 0][c], wd[p * MR_ROUND + j]);
+            }
+          }
+        } else {
+          for (int j = 0; j < jn; ++j) {  // a round with an infinite value
+            if ((starts >> j) & 1u) {
+              if (cur >= 0) lanes.flush(sre, sim, cur, m);
+              cur = __shfl_sync(0xffffffffu, key, j);
+            }
+#pragma unroll
+            for (int p = 0; p < NPOL; ++p)
+#pragma unroll
+              for (int c = 0; c < CPL; ++c) {
+                const int row = tr[(MULTI ? p : 0) * MR_ROUND + j], i = lane + 32 * c;
+                const int per = q.n_off * q.n_off;
+                int64_t at;
+                if (lanes.own[c] &&
+                    mosaic_tap(a, row / per, S, i / S, i % S, q.first + row / q.n_off % q.n_off,
+                               q.first + row % q.n_off, at))
+                  lanes.add(c, p, __ldg(a.cf + at), wd[p * MR_ROUND + j]);
+              }
+          }
+        }
+        __syncwarp();
+      }
+      if (cur >= 0) lanes.flush(sre, sim, cur, m);
+#pragma unroll
+      for (int p = 0; p < NPOL; ++p) {
+        double v = sw[p];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0 && a.sumw && lanes.ipm[p] >= 0 && v != 0.0)
+          atomicAdd(&a.sumw[plane * npg + lanes.ipm[p]], v);
+      }
+      __syncthreads();
+      // the segment's sub-grid to the global grid, a warp per row, cleared
+      for (int rr = warp; rr < npg * m.W; rr += MR_WARPS) {
+        const int gp = rr / m.W, iu = rr - gp * m.W;
+        double2 *gd = a.grid + ((plane * npg + gp) * a.n_u + (int64_t)tu * TILE + iu) * a.n_v +
+                      (int64_t)tv * TILE;
+        for (int iv = lane; iv < m.W; iv += 32) {
+          const int e = gp * m.PS + iu * m.RS + iv;
+          const double vr = sre[e], vi = sim[e];
+          if (vr == 0.0 && vi == 0.0) continue;
+          atomicAdd(&gd[iv].x, vr);
+          atomicAdd(&gd[iv].y, vi);
+          sre[e] = 0.0;
+          sim[e] = 0.0;
+        }
+      }
+      __syncthreads();
+      seg_lo = seg_hi;
+      if (seg_hi == t_end) ++tile;
+    }
+  }
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&t.sched[1], 1u) == gridDim.x - 1) {
+      t.sched[0] = 0u;
+      t.sched[1] = 0u;
+      __threadfence();
+    }
+  }
+}
+
+static int64_t mosaic_tap_rows(int64_t n_cf, int os) { return n_cf * (os + 1) * (os + 1); }
+
+static size_t mosaic_runs_smem(int S, int64_t n_img_pol, int npol_t) {
+  const size_t stage = (size_t)MR_WARPS * MR_ROUND * npol_t * (sizeof(double2) + sizeof(int));
+  return stage + (size_t)2 * n_img_pol * MosaicShape(S).PS * sizeof(double);
+}
+
+template <int CPL, int NPOL, bool MULTI>
+static int launch_mosaic_runs(const MosaicRunsArgs &q, int64_t n_chunks, cudaStream_t st) {
+  const size_t smem = mosaic_runs_smem(q.t.S, q.t.m.n_img_pol, NPOL);
+  auto kernel = k_mosaic_runs<CPL, NPOL, MULTI>;
+  AV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 1;
+  AV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, MR_THREADS, smem));
+  const int64_t most = (int64_t)sm_count() * std::max(per_sm, 1);
+  const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min(most, n_chunks));
+  kernel<<<blocks, MR_THREADS, smem, st>>>(q);
+  AV_LAUNCH_CHECK();
+  return AV_OK;
+}
+
+template <int CPL, int NPOL>
+static int launch_mosaic_runs(const MosaicRunsArgs &q, int64_t n_chunks, cudaStream_t st) {
+  // one tap row per sample when there is one function per (baseline, channel)
+  return q.t.m.n_cfp == 1 ? launch_mosaic_runs<CPL, NPOL, false>(q, n_chunks, st)
+                          : launch_mosaic_runs<CPL, NPOL, true>(q, n_chunks, st);
+}
+
+template <int CPL>
+static int launch_mosaic_runs(const MosaicRunsArgs &q, int64_t n_chunks, cudaStream_t st) {
+  if (q.t.m.npol <= 1) return launch_mosaic_runs<CPL, 1>(q, n_chunks, st);
+  if (q.t.m.npol <= 2) return launch_mosaic_runs<CPL, 2>(q, n_chunks, st);
+  return launch_mosaic_runs<CPL, 4>(q, n_chunks, st);
+}
+
 static size_t mosaic_tiled_smem(int S, int64_t n_img_pol) {
   const int W = TILE + S - 1;
   return (size_t)W * W * (size_t)n_img_pol * sizeof(double2);
@@ -747,6 +1150,80 @@ int av_mosaic_tiled_execute(AV_MOSAIC_PARAMS, void *workspace, size_t workspace_
   k_mosaic_tiled<<<(unsigned)nblocks, MT_THREADS, smem, as_stream(stream)>>>(t);
   AV_LAUNCH_CHECK();
   return AV_OK;
+}
+
+size_t av_mosaic_taps_size(int64_t n_cf, int max_support, int oversampling) {
+  if (n_cf < 1 || max_support < 1 || oversampling < 1) return 0;
+  const size_t rows = (size_t)mosaic_tap_rows(n_cf, oversampling);
+  return Workspace::need(rows * max_support * max_support * sizeof(double2)) +
+         Workspace::need(rows * sizeof(double));
+}
+
+int av_mosaic_runs_execute(AV_MOSAIC_PARAMS, void *workspace, size_t workspace_bytes, void *taps,
+                           size_t taps_bytes, void *stream) {
+  clear_error();
+  const char *who = "av_mosaic_runs_execute";
+  int rc = check_mosaic(who, grid, sum_weight, do_psf, vis, weight, uvw, freq, chan_map, pol_map,
+                        cf_baseline_map, cf_chan_map, cf_pol_map, cf, n_cf_baseline, n_cf_chan,
+                        n_cf_pol, conv_u, conv_v, support, max_support, n_u, n_v, delta_l,
+                        delta_m, os_u, os_v, nt, nb, nchan, npol, n_img_chan, n_img_pol);
+  if (rc) return rc;
+  AV_CHECK_ARG(os_u == os_v, "%s: oversampling must be the same on u, v", who);
+  AV_CHECK_ARG(n_img_pol <= 4 && npol <= 4, "%s: at most 4 polarisations", who);
+  AV_CHECK_ARG(max_support <= MR_MAX_S, "%s: max_support above %d", who, MR_MAX_S);
+  const int64_t n_cf = n_cf_baseline * n_cf_chan * n_cf_pol;
+  const int64_t rows_t = mosaic_tap_rows(n_cf, os_u);
+  AV_CHECK_ARG(rows_t <= 0x7fffffff, "%s: too many functions and offsets", who);
+  if (!taps || (((uintptr_t)taps) & 255) != 0 ||
+      taps_bytes < av_mosaic_taps_size(n_cf, max_support, os_u)) {
+    set_error("%s: tap workspace missing, misaligned or too small", who);
+    return AV_ERR_WORKSPACE;
+  }
+  PlanGeom g;
+  Plan p;
+  rc = mosaic_geom(g, p, n_u, n_v, max_support, os_u, nt, nb, nchan, n_img_chan, workspace,
+                   workspace_bytes, who);
+  if (rc) return rc;
+  const int64_t rows = nt * nb * nchan;
+  if (rows == 0 || npol == 0) return AV_OK;
+  MosaicRunsArgs q;
+  MosaicTiledArgs &t = q.t;
+  fill_mosaic(t.m, grid, sum_weight, do_psf, vis, weight, uvw, freq, chan_map, pol_map,
+              cf_baseline_map, cf_chan_map, cf_pol_map, cf, n_cf_baseline, n_cf_chan, n_cf_pol,
+              conv_u, conv_v, support, max_support, n_u, n_v, delta_l, delta_m, os_u, os_v, nt,
+              nb, nchan, npol, n_img_chan, n_img_pol);
+  t.recs = p.recs;
+  t.tile_start = p.tile_start;
+  t.n_rec = p.offs + g.n_keys();
+  t.sched = p.counters;
+  t.n_tiles = g.n_tiles();
+  t.ntu = g.ntu;
+  t.ntv = g.ntv;
+  t.S = max_support;
+  t.W = TILE + max_support - 1;
+  t.div_nchan = fast_div((uint32_t)nchan);
+  t.div_nb = fast_div((uint32_t)nb);
+  // a chunk per CTA slot and a few more to even out their times; at least
+  // 1024 records, so a chunk's sub-grid flush stays small against its samples
+  const int64_t parts = (int64_t)sm_count() * 16;
+  t.chunk = std::max<int64_t>(1024, (rows + parts - 1) / parts);
+  Workspace tw(taps, taps_bytes);
+  double2 *tab = tw.take<double2>((size_t)rows_t * max_support * max_support);
+  double *norm = tw.take<double>((size_t)rows_t);
+  q.taps = tab;
+  q.norm = norm;
+  // floor((u - u_pos) os + 0.5) with |u - u_pos| <= 0.5
+  q.first = -(os_u / 2);
+  q.n_off = os_u + 1;
+  cudaStream_t st = as_stream(stream);
+  k_mosaic_taps<<<(unsigned)rows_t, 128, 0, st>>>(t.m, max_support, q.first, q.n_off, tab, norm);
+  AV_LAUNCH_CHECK();
+  const int64_t n_chunks = (rows + t.chunk - 1) / t.chunk;
+  const int cpl = (max_support * max_support + 31) / 32;
+  if (cpl == 1) return launch_mosaic_runs<1>(q, n_chunks, st);
+  if (cpl == 2) return launch_mosaic_runs<2>(q, n_chunks, st);
+  if (cpl == 3) return launch_mosaic_runs<3>(q, n_chunks, st);
+  return launch_mosaic_runs<4>(q, n_chunks, st);
 }
 
 size_t av_aperture_grid_workspace_size(int64_t n_cf_baseline, int64_t nchan, int64_t npol) {

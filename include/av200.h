@@ -676,6 +676,23 @@ int av_mosaic_tiled_execute(void *grid, double *sum_weight, int do_psf, const vo
                             int64_t n_img_pol, void *workspace, size_t workspace_bytes,
                             void *stream);
 
+/* av_mosaic_tiled_execute for max_support <= 11 and npol <= 4, on the same
+ * plan, with each function's taps gathered by kernel offset into `taps`
+ * (256-byte aligned, av_mosaic_taps_size bytes; rewritten by every call) and
+ * the footprint's sums in registers. */
+size_t av_mosaic_taps_size(int64_t n_cf, int max_support, int oversampling);
+int av_mosaic_runs_execute(void *grid, double *sum_weight, int do_psf, const void *vis,
+                           const double *weight, const double *uvw, const double *freq,
+                           const int32_t *chan_map, const int32_t *pol_map,
+                           const int32_t *cf_baseline_map, const int32_t *cf_chan_map,
+                           const int32_t *cf_pol_map, const void *cf, int64_t n_cf_baseline,
+                           int64_t n_cf_chan, int64_t n_cf_pol, int64_t conv_u, int64_t conv_v,
+                           const int32_t *support, int max_support, int64_t n_u, int64_t n_v,
+                           double delta_l, double delta_m, int os_u, int os_v, int64_t nt,
+                           int64_t nb, int64_t nchan, int64_t npol, int64_t n_img_chan,
+                           int64_t n_img_pol, void *workspace, size_t workspace_bytes,
+                           void *taps, size_t taps_bytes, void *stream);
+
 /* aperture_grid_jit (mosaic_grid.py:13-153): every sample that passes the
  * grid-edge test adds weight x its function window at the grid centre
  * (and weight x Re(norm) to sum_weight); the weights are summed per

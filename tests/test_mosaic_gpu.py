@@ -214,3 +214,56 @@ def test_make_gridding_convolution_function_driver():
     with pytest.raises(AssertionError, match="gcf_params checking failed"):
         G.make_gridding_convolution_function(Dataset(), _duck_ms(g), dict(gcf_params,
                                              function="gauss"), grid_params, {})
+
+
+@pytest.mark.parametrize("max_support,os_", [(3, 4), (5, 5), (7, 4), (8, 3), (9, 10), (11, 4)])
+@pytest.mark.parametrize("npol,n_cfp", [(1, 1), (2, 1), (2, 2), (3, 3), (4, 1), (4, 2)])
+def test_register_mosaic_kernel(max_support, os_, npol, n_cfp):
+    """The kernel with the footprint in registers (windows up to 11 cells)
+    against the per-sample kernel: odd and even supports below the largest,
+    functions too small for their window, shared and separate polarisation
+    functions, maps with dropped entries, NaN, zero and infinite data, a grid
+    no tile divides.  Both add FP64 products of a few thousand samples in
+    another order: 1e-13 of the largest cell."""
+    import torch
+
+    from astroviper_b200 import _kernels as K
+    rng = np.random.default_rng(max_support * 100 + npol * 10 + n_cfp)
+    nt, nb, nchan, n_cfb, n_cfc = 35, 6, 3, 3, 2
+    n = (max_support + (0 if max_support == 7 else 1)) * os_
+    cf = rng.normal(size=(n_cfb, n_cfc, n_cfp, n, n)) + 1j * rng.normal(
+        size=(n_cfb, n_cfc, n_cfp, n, n))
+    sup = rng.integers(1, max_support + 1, size=(n_cfb, n_cfc, n_cfp, 2))
+    sup[0, 0, 0] = max_support
+    uvw = rng.normal(size=(nt, nb, 3)) * 500.0
+    uvw[0, 0, 0] = np.nan
+    vis = rng.normal(size=(nt, nb, nchan, npol)) + 1j * rng.normal(size=(nt, nb, nchan, npol))
+    wt = rng.uniform(0.5, 2.0, size=vis.shape)
+    wt[1] = 0.0
+    vis[2, 1] = np.nan
+    freq = np.array([1.0e9, 1.1e9, 1.3e9])
+    cell = np.array([-2.0, 2.0]) * np.pi / 180 / 3600 * 8
+    cfb, cfc, cm = np.array([0, 1, 2, 0, -1, 1]), np.array([0, 1, 1]), np.array([0, 1, 0])
+    pm, cfp = np.arange(npol)[::-1].copy(), np.arange(npol) % n_cfp
+    if npol == 3:
+        pm[1] = -1
+    for inf in (False, True):
+        if inf:
+            vis[3, 2, 1, 0] = np.inf
+        for do_psf in (False, True):
+            out = []
+            for tiled in (False, True):
+                grid = torch.zeros((2, npol, 101, 78), dtype=torch.complex128, device="cuda")
+                sw = torch.zeros((2, npol), dtype=torch.float64, device="cuda")
+                K.mosaic_grid(grid, sw, do_psf, vis, wt, uvw, freq, cm, pm, cfb, cfc, cfp,
+                              torch.as_tensor(cf, device="cuda"), sup, (101, 78), cell, os_,
+                              tiled=tiled)
+                out.append((grid.cpu().numpy(), sw.cpu().numpy()))
+            (ga, sa), (gb, sb) = out
+            assert np.array_equal(np.isfinite(ga), np.isfinite(gb))
+            ok = np.isfinite(ga)
+            assert np.abs(ga[ok]).max() > 0
+            assert np.abs(gb[ok] - ga[ok]).max() <= 1e-13 * np.abs(ga[ok]).max()
+            ok = np.isfinite(sa)
+            assert np.array_equal(ok, np.isfinite(sb))
+            assert np.abs(sb[ok] - sa[ok]).max() <= 1e-12 * np.abs(wt).sum() * max_support**2
