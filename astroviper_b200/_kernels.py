@@ -67,6 +67,15 @@ def on_device(x, dtype=None):
     return t.contiguous()
 
 
+def on_device_flag(flag):
+    """Contiguous uint8 CUDA tensor of a flag array (None stays None); a bool
+    array's bytes serve as they are."""
+    if flag is None:
+        return None
+    t = on_device(flag)
+    return t.view(torch.uint8) if t.dtype == torch.bool else t.to(torch.uint8).contiguous()
+
+
 # --------------------------------------------------------------------- PSWF --
 def pswf(u):
     u = on_device(u, torch.float64)
@@ -229,7 +238,7 @@ def degrid(grid_t, uvw, freq, scale, offset, chanmap, polmap, cgk, support, samp
     cm = on_device(chanmap, torch.int32)
     pm = on_device(polmap, torch.int32)
     cgk = on_device(cgk, torch.float64)
-    fl = None if flag is None else on_device(flag).to(torch.uint8).contiguous()
+    fl = on_device_flag(flag)
     dph = None if dphase is None else on_device(dphase, torch.float64)
     g_nchan, g_npol, g_n2, g_n3 = (int(s) for s in g.shape)
     tiled_ok = degrid_tiled_ok(precision, support, sampling, g_npol, c)
@@ -484,7 +493,7 @@ def weight_density(uvw, freq, weight, flag, n_uv, delta_lm, density=None, sum_we
     w = on_device(weight)
     if w.dtype not in (torch.float32, torch.float64):
         w = w.to(torch.float64)
-    fl = None if flag is None else on_device(flag).to(torch.uint8).contiguous()
+    fl = on_device_flag(flag)
     if density is None:
         density = torch.zeros((nchan, 1, nu, nv), dtype=torch.float64, device=dev)
     if sum_weight is None:
@@ -518,7 +527,7 @@ def briggs_apply(density, factors, uvw, freq, weight, flag, n_uv, delta_lm,
     w = on_device(weight)
     if w.dtype not in (torch.float32, torch.float64):
         w = w.to(torch.float64)
-    fl = None if flag is None else on_device(flag).to(torch.uint8).contiguous()
+    fl = on_device_flag(flag)
     out = torch.empty((nt, nb, nchan, npol), dtype=out_dtype, device=w.device)
     err = torch.zeros(1, dtype=torch.int32, device=w.device)
     dens_d = on_device(density, torch.float64)

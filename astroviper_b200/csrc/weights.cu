@@ -3,7 +3,9 @@
 // calculate_imaging_weights.py:183-198, 228-261).
 #include <math_constants.h>
 
+#include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -11,26 +13,29 @@ namespace av {
 
 // Polarisation-averaged weight of a sample, NaN where flagged
 // (calculate_imaging_weights.py:185-198).
-__device__ __forceinline__ double pol_avg_weight(const void *wt, int dt, const uint8_t *flag,
-                                                 int64_t row, int64_t npol) {
-  auto w = [&](int64_t p) {
-    int64_t i = row * npol + p;
-    double v = dt == AV_F32 ? (double)((const float *)wt)[i] : ((const double *)wt)[i];
+template <int NPOL, typename WT>
+__device__ __forceinline__ double pol_avg_weight(const WT *wt, const uint8_t *flag,
+                                                 int64_t row) {
+  auto w = [&](int p) {
+    const int64_t i = row * NPOL + p;
+    double v = (double)wt[i];
     if (flag && flag[i]) v = CUDART_NAN;
     return v;
   };
-  if (npol == 2) return __ddiv_rn(__dadd_rn(w(0), w(1)), 2.0);
-  if (npol == 4) return __ddiv_rn(__dadd_rn(w(0), w(3)), 2.0);
-  return w(0);
+  if (NPOL == 1) return w(0);
+  return __dmul_rn(__dadd_rn(w(0), w(NPOL - 1)), 0.5);  // the reference's / 2, exactly
 }
 
-// Nearest cell of a sample in the gridder's convention (int(x + 0.5)).
-__device__ __forceinline__ bool nearest_cell(double um, double vm, double f, double dl0,
-                                             double dl1, int64_t n_u, int64_t n_v,
-                                             long long &ui, long long &vi, long long &uic,
-                                             long long &vic) {
-  double us0 = __ddiv_rn(-__dmul_rn(__dmul_rn(f, dl0), (double)n_u), C_LIGHT);
-  double us1 = __ddiv_rn(-__dmul_rn(__dmul_rn(f, dl1), (double)n_v), C_LIGHT);
+// uv scale of a channel along one axis (standard_grid.py:297-299).
+__device__ __forceinline__ double uv_scale(double f, double dl, int64_t n) {
+  return __ddiv_rn(-__dmul_rn(__dmul_rn(f, dl), (double)n), C_LIGHT);
+}
+
+// Nearest cell of a sample in the gridder's convention (int(x + 0.5)), its
+// channel's scales given, and the cell of its conjugate.
+__device__ __forceinline__ bool scaled_cell(double um, double vm, double us0, double us1,
+                                            int64_t n_u, int64_t n_v, long long &ui,
+                                            long long &vi, long long &uic, long long &vic) {
   double u = __dmul_rn(um, us0), v = __dmul_rn(vm, us1);
   if (isnan(u) || isnan(v)) return false;
   double u_pos = __dadd_rn(u, (double)(n_u / 2)), v_pos = __dadd_rn(v, (double)(n_v / 2));
@@ -42,46 +47,117 @@ __device__ __forceinline__ bool nearest_cell(double um, double vm, double f, dou
   return (ui < n_u) && (vi < n_v) && (ui >= 0) && (vi >= 0);
 }
 
-// Density grid: rows enumerated channel-major so a warp shares a channel and
-// its sum_weight contribution is reduced before one atomic.
-__global__ void __launch_bounds__(256) k_weight_density(double *G, double *sumw,
-                                                        const double *uvw, const double *freq,
-                                                        const void *wt, int dt,
-                                                        const uint8_t *flag, int64_t n_u,
-                                                        int64_t n_v, double dl0, double dl1,
-                                                        int64_t ntb, int64_t nchan,
-                                                        int64_t npol) {
-  int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  int64_t total = ntb * nchan;
-  double add = 0.0;
-  int64_t c = -1;
-  if (k < total) {
-    c = k / ntb;
-    int64_t tb = k - c * ntb;
-    long long ui, vi, uic, vic;
-    if (nearest_cell(uvw[3 * tb], uvw[3 * tb + 1], freq[c], dl0, dl1, n_u, n_v, ui, vi, uic,
-                     vic)) {
-      double w = pol_avg_weight(wt, dt, flag, tb * nchan + c, npol);
-      if (!isnan(w)) {
-        double *plane = G + c * n_u * n_v;
-        atomicAdd(&plane[ui * n_v + vi], w);
+__device__ __forceinline__ bool nearest_cell(double um, double vm, double f, double dl0,
+                                             double dl1, int64_t n_u, int64_t n_v,
+                                             long long &ui, long long &vi, long long &uic,
+                                             long long &vic) {
+  return scaled_cell(um, vm, uv_scale(f, dl0, n_u), uv_scale(f, dl1, n_v), n_u, n_v, ui, vi, uic,
+                     vic);
+}
+
+// How k_weight_density and k_briggs_apply walk the samples: a thread takes
+// one (baseline, channel) series and `steps` consecutive times of it (grid:
+// series / WT_THREADS, time blocks).  At each time the threads of a warp read
+// neighbouring rows, whatever the number of channels; the channel's uv scale,
+// with its divides, is formed once; and since a baseline stays in one cell
+// for several times, its weights are summed in a register and its density
+// looked up once per cell.  WT_UNROLL times are loaded together (2 with 4 blocks
+// per SM: 47 and 54 us; 4 at once spill there, 57 and 69 us).
+constexpr int WT_THREADS = 256, WT_UNROLL = 2;
+
+// f(npol as a constant), npol 1, 2 or 4.
+template <typename F>
+static void with_pols(int64_t npol, F f) {
+  if (npol == 1) f(std::integral_constant<int, 1>());
+  else if (npol == 2) f(std::integral_constant<int, 2>());
+  else f(std::integral_constant<int, 4>());
+}
+
+static dim3 weight_walk(int64_t nt, int64_t series, int64_t &steps) {
+  // two waves of 1024 threads per SM, at least WT_UNROLL times each
+  const int64_t want = (int64_t)sm_count() * 2048;
+  const int64_t most = (nt + WT_UNROLL - 1) / WT_UNROLL;
+  int64_t blocks_t = std::max<int64_t>(1, std::min(most, (want + series - 1) / series));
+  blocks_t = std::min<int64_t>(blocks_t, 65535);
+  steps = (nt + blocks_t - 1) / blocks_t;
+  steps = (steps + WT_UNROLL - 1) / WT_UNROLL * WT_UNROLL;
+  blocks_t = (nt + steps - 1) / steps;
+  return dim3((unsigned)((series + WT_THREADS - 1) / WT_THREADS), (unsigned)blocks_t);
+}
+
+// Density grid and sums of weights.  One thread per sample in channel-major
+// order, two global FP64 atomics each and the weights read with a stride of a
+// whole row, had taken 270 us for 4.1M samples x 4 polarisations (float32,
+// 32 planes of 1024^2); this walk takes 47 us
+template <int NPOL, typename WT>
+__global__ void __launch_bounds__(WT_THREADS, 4) k_weight_density(
+    double *G, double *sumw, const double *__restrict__ uvw, const double *__restrict__ freq,
+    const WT *__restrict__ wt, const uint8_t *__restrict__ flag, int64_t n_u, int64_t n_v,
+    double dl0, double dl1, int64_t nt, int64_t nb, int64_t nchan, int64_t steps) {
+  __shared__ double s_sum[WT_THREADS];
+  const int64_t series = nb * nchan, s = blockIdx.x * (int64_t)WT_THREADS + threadIdx.x;
+  const bool shared_sum = nchan <= WT_THREADS;
+  s_sum[threadIdx.x] = 0.0;
+  __syncthreads();
+  double total = 0.0;
+  int64_t c = 0;
+  if (s < series) {
+    const int64_t b = s / nchan;
+    c = s - b * nchan;
+    const double us0 = uv_scale(freq[c], dl0, n_u), us1 = uv_scale(freq[c], dl1, n_v);
+    double *plane = G + c * n_u * n_v;
+    int64_t cell = -1, conj = -1;
+    double acc = 0.0;
+    auto flush = [&]() {
+      if (cell >= 0 && acc != 0.0) {
+        atomicAdd(plane + cell, acc);
         // the conjugate cell is not range-checked by the reference; it is out
         // of range only for index 0 of an even axis, skipped here
-        if (uic >= 0 && uic < n_u && vic >= 0 && vic < n_v) atomicAdd(&plane[uic * n_v + vic], w);
-        add = __dmul_rn(2.0, w);
+        if (conj >= 0) atomicAdd(plane + conj, acc);
+      }
+      acc = 0.0;
+    };
+    const int64_t t0 = blockIdx.y * steps, t1 = std::min(nt, t0 + steps);
+    for (int64_t t = t0; t < t1; t += WT_UNROLL) {
+      double um[WT_UNROLL], vm[WT_UNROLL], w[WT_UNROLL];
+#pragma unroll
+      for (int k = 0; k < WT_UNROLL; ++k)
+        if (t + k < t1) {
+          const int64_t tb = (t + k) * nb + b;
+          um[k] = uvw[3 * tb];
+          vm[k] = uvw[3 * tb + 1];
+          w[k] = pol_avg_weight<NPOL>(wt, flag, tb * nchan + c);
+        }
+#pragma unroll
+      for (int k = 0; k < WT_UNROLL; ++k) {
+        if (t + k >= t1) continue;
+        long long ui, vi, uic, vic;
+        if (!scaled_cell(um[k], vm[k], us0, us1, n_u, n_v, ui, vi, uic, vic) || isnan(w[k]))
+          continue;
+        const int64_t at = ui * n_v + vi;
+        const int64_t ac =
+            uic >= 0 && uic < n_u && vic >= 0 && vic < n_v ? uic * n_v + vic : -1;
+        if (at != cell || ac != conj) {
+          flush();
+          cell = at;
+          conj = ac;
+        }
+        acc += w[k];
+        total += __dmul_rn(2.0, w[k]);
       }
     }
+    flush();
   }
-  // lanes of a warp span at most two channels: the leader of each channel
-  // group sums the group's contributions and issues one atomic
-  int lane = threadIdx.x & 31;
-  unsigned m = __match_any_sync(0xffffffffu, (unsigned)(c + 1));
-  double tot = 0.0;
-  for (int l = 0; l < 32; ++l) {
-    double y = __shfl_sync(0xffffffffu, add, l);
-    if ((m >> l) & 1u) tot += y;
+  // sums of weights: one atomic per channel and block where a block's
+  // channels fit its threads
+  if (shared_sum) {
+    if (total != 0.0) atomicAdd(&s_sum[c], total);
+    __syncthreads();
+    if (threadIdx.x < nchan && s_sum[threadIdx.x] != 0.0)
+      atomicAdd(&sumw[threadIdx.x], s_sum[threadIdx.x]);
+  } else if (total != 0.0) {
+    atomicAdd(&sumw[c], total);
   }
-  if (lane == __ffs(m) - 1 && c >= 0 && tot != 0.0) atomicAdd(&sumw[c], tot);
 }
 
 // sum(G^2) per plane: one CTA per (plane, slice), FP64 partials.
@@ -110,53 +186,96 @@ __global__ void __launch_bounds__(256) k_sum_sq(const double *G, int64_t plane_n
   }
 }
 
-__global__ void k_briggs_finish(const double *partial, int slices, const double *sumw,
-                                int64_t nplanes, double robust, double *factors) {
-  int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// A warp per plane adds its partial sums (lane by lane, then in a tree: a
+// fixed order).
+__global__ void __launch_bounds__(128) k_briggs_finish(const double *partial, int slices,
+                                                       const double *sumw, int64_t nplanes,
+                                                       double robust, double *factors) {
+  const int lane = threadIdx.x & 31;
+  const int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   if (p >= nplanes) return;
   double sq = 0.0;
-  for (int s = 0; s < slices; ++s) sq += partial[p * slices + s];
+  for (int s = lane; s < slices; s += 32) sq += partial[p * slices + s];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+  if (lane != 0) return;
   double r = 5.0 * pow(10.0, -robust);
   // (5 * 10^-R)^2 / (sum G^2 / sum w): NaN / inf pass through like numpy
   factors[p] = (r * r) / (sq / sumw[p]);
   factors[nplanes + p] = 1.0;
 }
 
+template <typename T>
+struct PairOf {
+  using type = double2;
+};
+template <>
+struct PairOf<float> {
+  using type = float2;
+};
+
 // Imaging weight of each sample, tiled to every polarisation
-// (grid_imaging_weights.py:358-443 + calculate_imaging_weights.py:258-261).
-__global__ void __launch_bounds__(256) k_briggs_apply(void *out, int out_dt, const double *G,
-                                                      const double *factors, int64_t nplanes,
-                                                      const double *uvw, const double *freq,
-                                                      const void *wt, int dt,
-                                                      const uint8_t *flag, int64_t n_u,
-                                                      int64_t n_v, double dl0, double dl1,
-                                                      int64_t nrows, int64_t nchan,
-                                                      int64_t npol, int *err) {
-  int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (row >= nrows) return;
-  int64_t tb = row / nchan, c = row - tb * nchan;
-  double iw = 0.0;  // off-grid samples keep the zero the reference allocates
-  long long ui, vi, uic, vic;
-  if (nearest_cell(uvw[3 * tb], uvw[3 * tb + 1], freq[c], dl0, dl1, n_u, n_v, ui, vi, uic,
-                   vic)) {
-    double dw = pol_avg_weight(wt, dt, flag, row, npol);
-    iw = dw;
-    if (!isnan(dw) && dw != 0.0) {
-      double gij = G[(c * n_u + ui) * n_v + vi];
-      if (!isnan(gij) && gij != 0.0) {
-        double f0 = factors[c], f1 = factors[nplanes + c];
-        if (isnan(f0) || isnan(f1)) {
-          atomicExch(err, 1);
-        } else {
-          double denom = __dadd_rn(__dmul_rn(f0, gij), f1);
-          iw = __ddiv_rn(iw, denom);
+// (grid_imaging_weights.py:358-443 + calculate_imaging_weights.py:258-261),
+// in the walk above (89 us for the case above with one thread per sample;
+// 54 us now).
+template <int NPOL, typename OT, typename WT>
+__global__ void __launch_bounds__(WT_THREADS, 4) k_briggs_apply(
+    OT *out, const double *__restrict__ G, const double *__restrict__ factors, int64_t nplanes,
+    const double *__restrict__ uvw, const double *__restrict__ freq, const WT *__restrict__ wt,
+    const uint8_t *__restrict__ flag, int64_t n_u, int64_t n_v, double dl0, double dl1,
+    int64_t nt, int64_t nb, int64_t nchan, int64_t steps, int vec, int *err) {
+  const int64_t s = blockIdx.x * (int64_t)WT_THREADS + threadIdx.x;
+  if (s >= nb * nchan) return;
+  const int64_t b = s / nchan, c = s - b * nchan;
+  const double us0 = uv_scale(freq[c], dl0, n_u), us1 = uv_scale(freq[c], dl1, n_v);
+  const double f0 = factors[c], f1 = factors[nplanes + c];
+  const bool bad = isnan(f0) || isnan(f1);
+  const double *plane = G + c * n_u * n_v;
+  int64_t cell = -1;
+  double gij = 0.0;
+  const int64_t t0 = blockIdx.y * steps, t1 = std::min(nt, t0 + steps);
+  for (int64_t t = t0; t < t1; t += WT_UNROLL) {
+    double um[WT_UNROLL], vm[WT_UNROLL], dw[WT_UNROLL];
+#pragma unroll
+    for (int k = 0; k < WT_UNROLL; ++k)
+      if (t + k < t1) {
+        const int64_t tb = (t + k) * nb + b;
+        um[k] = uvw[3 * tb];
+        vm[k] = uvw[3 * tb + 1];
+        dw[k] = pol_avg_weight<NPOL>(wt, flag, tb * nchan + c);
+      }
+#pragma unroll
+    for (int k = 0; k < WT_UNROLL; ++k) {
+      if (t + k >= t1) continue;
+      double iw = 0.0;  // off-grid samples keep the zero the reference allocates
+      long long ui, vi, uic, vic;
+      if (scaled_cell(um[k], vm[k], us0, us1, n_u, n_v, ui, vi, uic, vic)) {
+        iw = dw[k];
+        if (!isnan(iw) && iw != 0.0) {
+          const int64_t at = ui * n_v + vi;
+          if (at != cell) {
+            cell = at;
+            gij = __ldg(plane + at);
+          }
+          if (!isnan(gij) && gij != 0.0) {
+            if (bad) atomicExch(err, 1);
+            else iw = __ddiv_rn(iw, __dadd_rn(__dmul_rn(f0, gij), f1));
+          }
         }
       }
+      OT *o = out + (((t + k) * nb + b) * nchan + c) * NPOL;
+      const OT v = (OT)iw;
+      if (NPOL > 1 && vec) {  // out is 16-byte aligned
+        using V = typename PairOf<OT>::type;
+        V pair;
+        pair.x = pair.y = v;
+#pragma unroll
+        for (int p = 0; p < NPOL; p += 2) *(V *)(o + p) = pair;
+      } else {
+#pragma unroll
+        for (int p = 0; p < NPOL; ++p) o[p] = v;
+      }
     }
-  }
-  for (int64_t p = 0; p < npol; ++p) {
-    if (out_dt == AV_F64) ((double *)out)[row * npol + p] = iw;
-    else ((float *)out)[row * npol + p] = (float)iw;
   }
 }
 
@@ -219,11 +338,18 @@ int av_weight_density(double *density, double *sum_weight, const double *uvw,
   AV_CHECK_ARG(npol == 1 || npol == 2 || npol == 4, "av_weight_density: npol must be 1, 2 or 4");
   AV_CHECK_ARG(n_u > 0 && n_v > 0 && nt >= 0 && nb >= 0 && nchan >= 0,
                "av_weight_density: bad shape");
-  int64_t total = nt * nb * nchan;
-  if (total == 0) return AV_OK;
-  k_weight_density<<<(unsigned)((total + 255) / 256), 256, 0, as_stream(stream)>>>(
-      density, sum_weight, uvw, freq, wt, wt_dtype, flag, n_u, n_v, delta_l, delta_m, nt * nb,
-      nchan, npol);
+  if (nt * nb * nchan == 0) return AV_OK;
+  int64_t steps = 0;
+  const dim3 grid = weight_walk(nt, nb * nchan, steps);
+  auto run = [&](auto pol, const auto *w) {
+    k_weight_density<decltype(pol)::value><<<grid, WT_THREADS, 0, as_stream(stream)>>>(
+        density, sum_weight, uvw, freq, w, flag, n_u, n_v, delta_l, delta_m, nt, nb, nchan,
+        steps);
+  };
+  with_pols(npol, [&](auto pol) {
+    if (wt_dtype == AV_F32) run(pol, (const float *)wt);
+    else run(pol, (const double *)wt);
+  });
   AV_LAUNCH_CHECK();
   return AV_OK;
 }
@@ -248,7 +374,7 @@ int av_briggs_factors(const double *density, const double *sum_weight, double *f
   double *partial = (double *)workspace;
   k_sum_sq<<<(unsigned)(nplanes * slices), 256, 0, st>>>(density, n_u * n_v, slices, partial);
   AV_LAUNCH_CHECK();
-  k_briggs_finish<<<(unsigned)((nplanes + 127) / 128), 128, 0, st>>>(partial, slices,
+  k_briggs_finish<<<(unsigned)((nplanes + 3) / 4), 128, 0, st>>>(partial, slices,
                                                                       sum_weight, nplanes,
                                                                       robust, factors);
   AV_LAUNCH_CHECK();
@@ -266,12 +392,21 @@ int av_briggs_apply(void *out, int out_dtype, const double *density, const doubl
   AV_CHECK_ARG(out_dtype == AV_F32 || out_dtype == AV_F64, "av_briggs_apply: out dtype");
   AV_CHECK_ARG(wt_dtype == AV_F32 || wt_dtype == AV_F64, "av_briggs_apply: weight dtype");
   AV_CHECK_ARG(npol == 1 || npol == 2 || npol == 4, "av_briggs_apply: npol must be 1, 2 or 4");
-  int64_t rows = nt * nb * nchan;
-  if (rows == 0) return AV_OK;
-  cudaStream_t st = as_stream(stream);
-  k_briggs_apply<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(
-      out, out_dtype, density, factors, nchan, uvw, freq, wt, wt_dtype, flag, n_u, n_v, delta_l,
-      delta_m, rows, nchan, npol, err_flag);
+  if (nt * nb * nchan == 0) return AV_OK;
+  int64_t steps = 0;
+  const dim3 grid = weight_walk(nt, nb * nchan, steps);
+  const int vec = (((uintptr_t)out) & 15) == 0;
+  auto run = [&](auto pol, auto *o, const auto *w) {
+    k_briggs_apply<decltype(pol)::value><<<grid, WT_THREADS, 0, as_stream(stream)>>>(
+        o, density, factors, nchan, uvw, freq, w, flag, n_u, n_v, delta_l, delta_m, nt, nb, nchan,
+        steps, vec, err_flag);
+  };
+  with_pols(npol, [&](auto pol) {
+    if (out_dtype == AV_F64 && wt_dtype == AV_F64) run(pol, (double *)out, (const double *)wt);
+    else if (out_dtype == AV_F64) run(pol, (double *)out, (const float *)wt);
+    else if (wt_dtype == AV_F64) run(pol, (float *)out, (const double *)wt);
+    else run(pol, (float *)out, (const float *)wt);
+  });
   AV_LAUNCH_CHECK();
   return AV_OK;
 }

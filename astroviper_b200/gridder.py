@@ -208,7 +208,7 @@ class Gridder:
                                  dtype=torch.complex64, device=self.dev)
             accumulate = False
         pm = self._degrid_polmap(g_npol)
-        fl = None if flag is None else K.on_device(flag).to(torch.uint8).contiguous()
+        fl = K.on_device_flag(flag)
         dph = None if dphase is None else K.on_device(dphase, torch.float64)
         check(lib().av_degrid_tiled_execute(K.p(dph), K.p(values), K.dcode(values),
                                             int(bool(accumulate)), K.p(fl),
