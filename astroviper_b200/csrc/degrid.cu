@@ -188,7 +188,7 @@ constexpr int DT_THREADS = 256;
 struct TiledDegridArgs {
   const Rec *recs;
   const uint32_t *tile_start;
-  const uint32_t *n_rec;    // device: usable records (offs[n_keys])
+  const uint32_t *n_rec;    // device: usable records
   const uint32_t *exc_mark; // device: a shared plan's marks (zero otherwise)
   int64_t n_rows;           // all samples (the plan also lists skipped ones)
   int64_t n_tiles, ntu, ntv, chunk;
@@ -1826,7 +1826,7 @@ int av_degrid_tiled_execute(const double *dphase, void *values, int values_dtype
   TiledDegridArgs a;
   a.recs = p.recs;
   a.tile_start = p.tile_start;
-  a.n_rec = p.offs + g.n_keys();
+  a.n_rec = p.n_rec;
   a.exc_mark = p.exc_mark;
   a.n_tiles = g.n_tiles();
   a.ntu = g.ntu;
@@ -1929,7 +1929,7 @@ int av_degrid_double(const double *uvw, const double *dphase, void *values, int 
   if (rc) return rc;
   a.recs = p.recs;
   a.tile_start = p.tile_start;
-  a.n_rec = p.offs + g.n_keys();
+  a.n_rec = p.n_rec;
   a.n_tiles = g.n_tiles();
   a.ntu = g.ntu;
   a.ntv = g.ntv;

@@ -162,7 +162,7 @@ constexpr int GT_STAGE = 32;  // samples a warp stages per round (one per lane)
 struct TiledGridArgs {
   const Rec *recs;
   const uint32_t *tile_start;
-  const uint32_t *n_rec;  // device: total records (offs[n_keys])
+  const uint32_t *n_rec;  // device: usable records
   uint32_t *sched;        // device: [0] next chunk, [1] CTAs done (both 0 between launches)
   int a16;                 // vis and weight rows are 16-byte aligned (16-byte loads / copies)
   int64_t n_tiles, ntu, ntv;
@@ -1539,7 +1539,7 @@ int av_tiled_plan_counts(int64_t nt, int64_t nb, int64_t nchan, int64_t n_u, int
                              (void *)workspace, workspace_bytes, p, "av_tiled_plan_counts");
   if (rc) return rc;
   cudaStream_t st = as_stream(stream);
-  AV_CUDA(cudaMemcpyAsync(&out[0], p.offs + g.n_keys(), sizeof(uint32_t), cudaMemcpyDeviceToHost,
+  AV_CUDA(cudaMemcpyAsync(&out[0], p.n_rec, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                           st));
   AV_CUDA(cudaMemcpyAsync(&out[1], p.exc_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   AV_CUDA(cudaStreamSynchronize(st));
@@ -1564,7 +1564,7 @@ static int grid_execute(const char *who, void *grid, int grid_dtype, double *sum
   TiledGridArgs a;
   a.recs = p.recs;
   a.tile_start = p.tile_start;
-  a.n_rec = p.offs + g.n_keys();
+  a.n_rec = p.n_rec;
   a.n_tiles = g.n_tiles();
   a.ntu = g.ntu;
   a.ntv = g.ntv;
@@ -1691,7 +1691,7 @@ int av_grid_tiled_execute_det(void *grid, int grid_dtype, double *sum_weight, in
   TiledGridArgs a;
   a.recs = p.recs;
   a.tile_start = p.tile_start;
-  a.n_rec = p.offs + g.n_keys();
+  a.n_rec = p.n_rec;
   a.n_tiles = g.n_tiles();
   a.ntu = g.ntu;
   a.ntv = g.ntv;
@@ -1798,7 +1798,7 @@ int av_degrid_tiled_adjoint(void *grid, int grid_dtype, const void *values, int 
   TiledGridArgs a;
   a.recs = p.recs;
   a.tile_start = p.tile_start;
-  a.n_rec = p.offs + g.n_keys();
+  a.n_rec = p.n_rec;
   a.n_tiles = g.n_tiles();
   a.ntu = g.ntu;
   a.ntv = g.ntv;

@@ -1128,7 +1128,7 @@ int av_mosaic_tiled_execute(AV_MOSAIC_PARAMS, void *workspace, size_t workspace_
               nb, nchan, npol, n_img_chan, n_img_pol);
   t.recs = p.recs;
   t.tile_start = p.tile_start;
-  t.n_rec = p.offs + g.n_keys();
+  t.n_rec = p.n_rec;
   t.sched = p.counters;
   t.n_tiles = g.n_tiles();
   t.ntu = g.ntu;
@@ -1194,7 +1194,7 @@ int av_mosaic_runs_execute(AV_MOSAIC_PARAMS, void *workspace, size_t workspace_b
               nb, nchan, npol, n_img_chan, n_img_pol);
   t.recs = p.recs;
   t.tile_start = p.tile_start;
-  t.n_rec = p.offs + g.n_keys();
+  t.n_rec = p.n_rec;
   t.sched = p.counters;
   t.n_tiles = g.n_tiles();
   t.ntu = g.ntu;

@@ -3,16 +3,6 @@
 
 namespace av {
 
-// Per-channel uv scale of the gridder: -(f * dl * n) / c (standard_grid.py:297-299).
-__global__ void k_chan_scale(const double *freq, int64_t nchan, double dl0, double dl1,
-                             int64_t n_u, int64_t n_v, double *scale) {
-  int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c >= nchan) return;
-  double f = freq[c];
-  scale[2 * c + 0] = __ddiv_rn(-__dmul_rn(__dmul_rn(f, dl0), (double)n_u), C_LIGHT);
-  scale[2 * c + 1] = __ddiv_rn(-__dmul_rn(__dmul_rn(f, dl1), (double)n_v), C_LIGHT);
-}
-
 // Work units of the two passes: unit u = (baseline b, block of 32 time
 // steps), lane = time step inside the block.  A warp takes units u, u +
 // n_warps, ... and walks the unit's channels one after the other, so the
@@ -275,10 +265,18 @@ __global__ void __launch_bounds__(256) k_plan_scatter(PlanGeom g,
 }
 
 // --------------------------------------------------------------- scan ------
-// Exclusive scan of n uint32 values in place into out (n + 1 entries; out[n]
-// = total), three phases with 4096 items per block.
+// Exclusive scan of the key counts in place (n uint32 values, 16-byte
+// aligned), SCAN_TILE of them per block: the blocks' sums, then each block's
+// own scan from the sum of the sums before it.  A block adds those up itself
+// while there are at most SCAN_SELF of them (4 loads a thread); for more, a
+// pass in between scans them.  The second pass also writes the total, the
+// tile starts (every kpt-th value) and zeroes the scheduling counters, and
+// the scatter pass turns each start into its key's end, so no second array of
+// key starts is written.  16-byte accesses: 14M keys take 48 us, 102
+// with 4-byte ones, a second array and separate passes.
 constexpr int SCAN_BLK = 1024, SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_BLK * SCAN_ITEMS;
+constexpr int64_t SCAN_SELF = 4096;
 
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *sh,
                                                          uint32_t &total) {
@@ -308,17 +306,27 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s
   return r;
 }
 
+// Items base .. base + 3 (zeros past n).
+__device__ __forceinline__ uint4 scan_load(const uint32_t *x, int64_t base, int64_t n) {
+  if (base + SCAN_ITEMS <= n) return *(const uint4 *)(x + base);
+  uint4 v = make_uint4(0u, 0u, 0u, 0u);
+  if (base < n) v.x = x[base];
+  if (base + 1 < n) v.y = x[base + 1];
+  if (base + 2 < n) v.z = x[base + 2];
+  return v;
+}
+
 __global__ void __launch_bounds__(SCAN_BLK) k_scan_reduce(const uint32_t *in, int64_t n,
                                                           uint32_t *partial) {
   __shared__ uint32_t sh[32];
-  int64_t base = blockIdx.x * (int64_t)SCAN_TILE + threadIdx.x * SCAN_ITEMS;
-  uint32_t s = 0;
-#pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k)
-    if (base + k < n) s += in[base + k];
-  uint32_t total;
-  block_exclusive_scan(s, sh, total);
-  if (threadIdx.x == 0) partial[blockIdx.x] = total;
+  const uint4 v = scan_load(in, blockIdx.x * (int64_t)SCAN_TILE + threadIdx.x * SCAN_ITEMS, n);
+  const uint32_t w = __reduce_add_sync(0xffffffffu, v.x + v.y + v.z + v.w);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = w;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const uint32_t t = __reduce_add_sync(0xffffffffu, sh[threadIdx.x]);
+    if (threadIdx.x == 0) partial[blockIdx.x] = t;
+  }
 }
 
 __global__ void __launch_bounds__(SCAN_BLK) k_scan_partials(uint32_t *partial, int64_t np) {
@@ -338,56 +346,86 @@ __global__ void __launch_bounds__(SCAN_BLK) k_scan_partials(uint32_t *partial, i
   }
 }
 
-__global__ void __launch_bounds__(SCAN_BLK) k_scan_final(const uint32_t *in, int64_t n,
-                                                         const uint32_t *partial,
-                                                         uint32_t *out, uint32_t *out2) {
-  __shared__ uint32_t sh[32];
-  int64_t base = blockIdx.x * (int64_t)SCAN_TILE + threadIdx.x * SCAN_ITEMS;
-  uint32_t v[SCAN_ITEMS];
-  uint32_t s = 0;
-#pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k) {
-    v[k] = (base + k < n) ? in[base + k] : 0;
-    s += v[k];
-  }
-  uint32_t total;
-  uint32_t ex = block_exclusive_scan(s, sh, total) + partial[blockIdx.x];
-#pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k) {
-    if (base + k < n) {
-      out[base + k] = ex;
-      out2[base + k] = ex;
+// x: counts in, key starts out (in place); *n_rec: the last key's start, the
+// number of usable records; tile_start[t] = the start of key t << kpt_shift;
+// counters: zeroed.  `scanned`: partial
+// holds the blocks' exclusive prefixes, else their sums.
+__global__ void __launch_bounds__(SCAN_BLK) k_scan_final(uint32_t *x, int64_t n,
+                                                         const uint32_t *partial, int scanned,
+                                                         uint32_t *n_rec, int kpt_shift,
+                                                         uint32_t *tile_start,
+                                                         uint32_t *counters) {
+  __shared__ uint32_t sh[32], s_before;
+  if (blockIdx.x == 0 && threadIdx.x < 16) counters[threadIdx.x] = 0u;
+  const int64_t base = blockIdx.x * (int64_t)SCAN_TILE + threadIdx.x * SCAN_ITEMS;
+  const uint4 v = scan_load(x, base, n);
+  uint32_t before;
+  if (scanned) {
+    before = partial[blockIdx.x];
+  } else {
+    uint32_t s = 0;
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += SCAN_BLK) s += partial[k];
+    s = __reduce_add_sync(0xffffffffu, s);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      s = __reduce_add_sync(0xffffffffu, sh[threadIdx.x]);
+      if (threadIdx.x == 0) s_before = s;
     }
-    ex += v[k];
+    __syncthreads();
+    before = s_before;
   }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) {
-    out[n] = ex;
-    out2[n] = ex;
+  uint32_t all;
+  uint4 e;
+  e.x = before + block_exclusive_scan(v.x + v.y + v.z + v.w, sh, all);
+  e.y = e.x + v.x;
+  e.z = e.y + v.y;
+  e.w = e.z + v.z;
+  const uint32_t ex[SCAN_ITEMS] = {e.x, e.y, e.z, e.w};
+  if (base + SCAN_ITEMS <= n) {
+    *(uint4 *)(x + base) = e;
+  } else {
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; ++k)
+      if (base + k < n) x[base + k] = ex[k];
   }
+  const int64_t mask = ((int64_t)1 << kpt_shift) - 1;
+#pragma unroll
+  for (int k = 0; k < SCAN_ITEMS; ++k)
+    if (base + k < n && ((base + k) & mask) == 0) tile_start[(base + k) >> kpt_shift] = ex[k];
+#pragma unroll
+  for (int k = 0; k < SCAN_ITEMS; ++k)
+    if (base + k == n - 1) *n_rec = ex[k];
 }
 
-// Scan of counts held in `cursor` into offs (and a copy back into cursor to
-// serve as the scatter cursors).
-static int scan_counts(uint32_t *counts_then_cursor, uint32_t *offs, int64_t n,
-                       uint32_t *tmp, cudaStream_t st) {
+// Turns the counts of n keys (the last one the skipped samples') into starts
+// in place.
+static int scan_counts(const PlanGeom &g, const Plan &p, int64_t n, cudaStream_t st) {
   int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
   if (nb < 1) nb = 1;
   if (nb > SCAN_MAX_BLOCKS) {
     set_error("plan: key count %lld exceeds the scan capacity", (long long)n);
     return AV_ERR_UNSUPPORTED;
   }
-  k_scan_reduce<<<(unsigned)nb, SCAN_BLK, 0, st>>>(counts_then_cursor, n, tmp);
+  k_scan_reduce<<<(unsigned)nb, SCAN_BLK, 0, st>>>(p.cursor, n, p.scan_tmp);
   AV_LAUNCH_CHECK();
-  k_scan_partials<<<1, SCAN_BLK, 0, st>>>(tmp, nb);
-  AV_LAUNCH_CHECK();
-  k_scan_final<<<(unsigned)nb, SCAN_BLK, 0, st>>>(counts_then_cursor, n, tmp, offs,
-                                                   counts_then_cursor);
+  const int scanned = nb > SCAN_SELF;
+  if (scanned) {
+    k_scan_partials<<<1, SCAN_BLK, 0, st>>>(p.scan_tmp, nb);
+    AV_LAUNCH_CHECK();
+  }
+  int kpt_shift = 0;
+  while (((int64_t)1 << kpt_shift) < g.kpt) ++kpt_shift;
+  k_scan_final<<<(unsigned)nb, SCAN_BLK, 0, st>>>(p.cursor, n, p.scan_tmp, scanned,
+                                                   p.n_rec, kpt_shift, p.tile_start,
+                                                   p.counters);
   AV_LAUNCH_CHECK();
   return AV_OK;
 }
 
 // ------------------------------------------------------------- row order ---
-// For deterministic gridding (av_grid_tiled_execute_det): each key's records
+// For deterministic gridding (av_grid_tiled_execute_det), after the scatter
+// pass has left every key's end in cursor (`ends`): each key's records
 // ordered by row, so the order in which a cell's samples are summed is a
 // property of the data, not of the scatter pass's atomics.  Keys of up to
 // ORD_WCAP records are sorted by one warp in shared memory, keys of up to
@@ -458,7 +496,7 @@ __device__ __forceinline__ void put_rec(Rec *recs, uint32_t *exc_mark, uint32_t 
   recs[pos] = r;
 }
 
-__global__ void __launch_bounds__(ROW_WARPS * 32) k_plan_order_rows(const uint32_t *offs,
+__global__ void __launch_bounds__(ROW_WARPS * 32) k_plan_order_rows(const uint32_t *ends,
                                                                     int64_t n_keys, Rec *recs,
                                                                     uint32_t *exc_mark,
                                                                     uint32_t *big,
@@ -471,8 +509,8 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) k_plan_order_rows(const uint32
     const int64_t k = k0 + lane;
     uint32_t lo = 0, n = 0;
     if (k < n_keys) {
-      lo = offs[k];
-      n = offs[k + 1] - lo;
+      lo = k ? ends[k - 1] : 0u;
+      n = ends[k] - lo;
     }
     if (n > (uint32_t)ORD_WCAP) big[atomicAdd(n_big, 1u)] = (uint32_t)k;
     unsigned todo = __ballot_sync(0xffffffffu, n >= 2 && n <= (uint32_t)ORD_WCAP);
@@ -490,7 +528,7 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) k_plan_order_rows(const uint32
   }
 }
 
-__global__ void __launch_bounds__(ROW_BTHREADS) k_plan_order_rows_big(const uint32_t *offs,
+__global__ void __launch_bounds__(ROW_BTHREADS) k_plan_order_rows_big(const uint32_t *ends,
                                                                       Rec *recs,
                                                                       uint32_t *exc_mark,
                                                                       const uint32_t *big,
@@ -504,7 +542,7 @@ __global__ void __launch_bounds__(ROW_BTHREADS) k_plan_order_rows_big(const uint
   if (blockIdx.x == 0 && threadIdx.x == 0) plan_counters[PLAN_ROWS_ORDERED] = 1u;
   for (uint32_t it = blockIdx.x; it < nb; it += gridDim.x) {
     const uint32_t k = big[it];
-    const uint32_t lo = offs[k], n = offs[k + 1] - lo;
+    const uint32_t lo = k ? ends[k - 1] : 0u, n = ends[k] - lo;
     const bool in_smem = n <= (uint32_t)ROW_BCAP;  // uniform over the CTA
     if (in_smem) {
       for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
@@ -544,31 +582,22 @@ int plan_order_rows(const PlanGeom &g, const Plan &p, cudaStream_t st) {
   AV_CUDA(cudaMemsetAsync(p.n_big, 0, sizeof(uint32_t), st));
   int64_t blocks = (nk + ROW_WARPS * 32 - 1) / (ROW_WARPS * 32);
   if (blocks > (int64_t)sms * 3) blocks = (int64_t)sms * 3;
-  k_plan_order_rows<<<(unsigned)blocks, ROW_WARPS * 32, ROW_SMEM, st>>>(p.offs, nk, p.recs,
+  k_plan_order_rows<<<(unsigned)blocks, ROW_WARPS * 32, ROW_SMEM, st>>>(p.cursor, nk, p.recs,
                                                                        p.exc_mark, p.big,
                                                                        p.n_big);
   AV_LAUNCH_CHECK();
-  k_plan_order_rows_big<<<(unsigned)sms, ROW_BTHREADS, ROW_BSMEM, st>>>(p.offs, p.recs,
+  k_plan_order_rows_big<<<(unsigned)sms, ROW_BTHREADS, ROW_BSMEM, st>>>(p.cursor, p.recs,
                                                                         p.exc_mark, p.big,
                                                                         p.n_big, p.counters);
   AV_LAUNCH_CHECK();
   return AV_OK;
 }
 
-// Tile starts, and the plan's scheduling counters set to zero (the tiled
-// kernels take chunks from them and leave them at zero when they finish).
-__global__ void k_tile_starts(const uint32_t *offs, int64_t n_tiles, int64_t kpt,
-                              uint32_t *tile_start, uint32_t *counters) {
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t < 16) counters[t] = 0u;
-  if (t > n_tiles) return;
-  tile_start[t] = offs[t * kpt];
-}
-
 // Zeroes the cells a plan's records can touch: the (TILE + support - 1)^2
 // footprint region of every tile that holds records, all grid polarisations
-// (one CTA per tile; empty tiles return at once).  Neighbouring regions
-// overlap; they all write zero.
+// (one CTA per tile, a warp per row; empty tiles return at once).
+// Neighbouring regions overlap; they all write zero.  128 grids of 1024^2:
+// 68 us, against 105 with an element's place divided out each time.
 __global__ void __launch_bounds__(256) k_clear_tiles(const uint32_t *tile_start, PlanGeom g,
                                                      void *grid, int grid_c128, int64_t npg) {
   const int64_t t = blockIdx.x;
@@ -576,15 +605,17 @@ __global__ void __launch_bounds__(256) k_clear_tiles(const uint32_t *tile_start,
   const int64_t plane = t / (g.ntu * g.ntv);
   const int64_t trem = t - plane * g.ntu * g.ntv;
   const int64_t tu = trem / g.ntv, tv = trem - tu * g.ntv;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int W = TILE + g.support - 1;
-  const int64_t n = (int64_t)W * W * npg;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const int64_t gp = i / ((int64_t)W * W), cell = i - gp * W * W;
-    const int64_t gu = tu * TILE + cell / W, gv = tv * TILE + cell % W;
-    if (gu >= g.n_u || gv >= g.n_v) continue;
-    const int64_t gi = ((plane * npg + gp) * g.n_u + gu) * g.n_v + gv;
-    if (grid_c128) ((double2 *)grid)[gi] = make_double2(0.0, 0.0);
-    else ((float2 *)grid)[gi] = make_float2(0.f, 0.f);
+  const int wu = (int)min((int64_t)W, g.n_u - tu * TILE), wv = (int)min((int64_t)W, g.n_v - tv * TILE);
+  for (int64_t gp = 0; gp < npg; ++gp) {
+    const int64_t corner = ((plane * npg + gp) * g.n_u + tu * TILE) * g.n_v + tv * TILE;
+    for (int iu = warp; iu < wu; iu += warps)
+      for (int iv = lane; iv < wv; iv += 32) {
+        const int64_t gi = corner + iu * g.n_v + iv;
+        if (grid_c128) ((double2 *)grid)[gi] = make_double2(0.0, 0.0);
+        else ((float2 *)grid)[gi] = make_float2(0.f, 0.f);
+      }
   }
 }
 
@@ -597,7 +628,7 @@ int plan_clear_tiles(const PlanGeom &g, const Plan &p, void *grid, int grid_c128
 }
 
 bool plan_carve(const PlanGeom &g, Workspace &ws, Plan &p) {
-  p.offs = ws.take<uint32_t>(g.n_keys() + 2);
+  p.n_rec = ws.take<uint32_t>(4);
   p.cursor = ws.take<uint32_t>(g.n_keys() + 2);
   p.tile_start = ws.take<uint32_t>(g.n_tiles() + 1);
   p.recs = ws.take<Rec>(g.n_rows > 0 ? g.n_rows : 1);
@@ -615,30 +646,49 @@ bool plan_carve(const PlanGeom &g, Workspace &ws, Plan &p) {
   p.freq = ws.take<double>(g.nchan > 0 ? g.nchan : 1);
   p.chan_map = ws.take<int32_t>(g.nchan > 0 ? g.nchan : 1);
   p.dpar = ws.take<double>(4);
-  return p.offs && p.cursor && p.tile_start && p.recs && p.scale && p.scan_tmp &&
+  return p.n_rec && p.cursor && p.tile_start && p.recs && p.scale && p.scan_tmp &&
          p.counters && p.walk_key && p.walk_rec && p.exc_count && p.exc_rows && p.exc_mark &&
          p.n_big && p.big && p.uv &&
          p.freq && p.chan_map && p.dpar;
 }
 
-// What the exception kernel of a shared plan reads: u, v of every (time,
-// baseline), the frequencies, the channel map and the degridder's scale /
-// offset (so the plan stands on its own after the caller's arrays change).
-__global__ void k_shared_copy(const double *uvw, int64_t ntb, const double *freq,
-                              const int32_t *chan_map, int64_t nchan, double s0, double s1,
-                              double o0, double o1, double2 *uv, double *fcopy, int32_t *ccopy,
-                              double *dpar) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < ntb) uv[i] = make_double2(uvw[3 * i], uvw[3 * i + 1]);
-  if (i < nchan) {
-    fcopy[i] = freq[i];
-    ccopy[i] = chan_map[i];
+// Everything a build starts from, in one launch where there were three clears
+// and two kernels: key counts, exception count and marks zeroed, the
+// gridder's uv scale of each channel, -(f * dl * n) / c
+// (standard_grid.py:297-299), and, for a shared plan, what its exception
+// kernel reads: u, v of every (time, baseline), the frequencies, the channel
+// map and the degridder's scale / offset (so the plan stands on its own after
+// the caller's arrays change).
+__global__ void __launch_bounds__(256) k_plan_setup(PlanGeom g, Plan p,
+                                                    const double *__restrict__ uvw,
+                                                    const double *__restrict__ freq,
+                                                    const int32_t *__restrict__ chan_map,
+                                                    double dl0, double dl1) {
+  const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t words = g.n_keys() + 2, quads = words / 4;  // 256-byte aligned
+  for (int64_t i = first; i < quads; i += stride) ((uint4 *)p.cursor)[i] = make_uint4(0, 0, 0, 0);
+  if (first < words - quads * 4) p.cursor[quads * 4 + first] = 0u;
+  const int64_t marks = (g.n_rows > 0 ? g.n_rows : 1) / 32 + 2;
+  for (int64_t i = first; i < marks; i += stride) p.exc_mark[i] = 0u;
+  if (first < 4) p.exc_count[first] = 0u;
+  for (int64_t c = first; c < g.nchan; c += stride) {
+    const double f = freq[c];
+    p.scale[2 * c + 0] = __ddiv_rn(-__dmul_rn(__dmul_rn(f, dl0), (double)g.n_u), C_LIGHT);
+    p.scale[2 * c + 1] = __ddiv_rn(-__dmul_rn(__dmul_rn(f, dl1), (double)g.n_v), C_LIGHT);
+    if (g.convention == 2) {
+      p.freq[c] = f;
+      p.chan_map[c] = chan_map[c];
+    }
   }
-  if (i == 0) {
-    dpar[0] = s0;
-    dpar[1] = s1;
-    dpar[2] = o0;
-    dpar[3] = o1;
+  if (g.convention != 2) return;
+  for (int64_t i = first; i < g.nt * g.nb; i += stride)
+    p.uv[i] = make_double2(uvw[3 * i], uvw[3 * i + 1]);
+  if (first == 0) {
+    p.dpar[0] = g.scale0;
+    p.dpar[1] = g.scale1;
+    p.dpar[2] = g.offset0;
+    p.dpar[3] = g.offset1;
   }
 }
 
@@ -655,25 +705,13 @@ int plan_build(const PlanGeom &g, Plan &p, const double *uvw, const double *freq
     set_error("plan: %lld samples exceed a shared plan's 31-bit rows", (long long)g.n_rows);
     return AV_ERR_UNSUPPORTED;
   }
-  AV_CUDA(cudaMemsetAsync(p.cursor, 0, sizeof(uint32_t) * (nk + 2), st));
-  AV_CUDA(cudaMemsetAsync(p.exc_count, 0, sizeof(uint32_t) * 4, st));
-  AV_CUDA(cudaMemsetAsync(p.exc_mark, 0,
-                          sizeof(uint32_t) * ((g.n_rows > 0 ? g.n_rows : 1) / 32 + 2), st));
-  if (g.convention == 2) {
-    const int64_t n = std::max<int64_t>(g.nt * g.nb, g.nchan);
-    if (n > 0) {
-      k_shared_copy<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
-          uvw, g.nt * g.nb, freq, chan_map, g.nchan, g.scale0, g.scale1, g.offset0, g.offset1,
-          p.uv, p.freq, p.chan_map, p.dpar);
-      AV_LAUNCH_CHECK();
-    }
-  }
-  if (g.nchan > 0) {
-    k_chan_scale<<<(unsigned)((g.nchan + 127) / 128), 128, 0, st>>>(
-        freq, g.nchan, delta_l, delta_m, g.n_u, g.n_v, p.scale);
+  int sms = sm_count();
+  {
+    const int64_t most = std::max(nk / 4, std::max(g.nt * g.nb, std::max(g.nchan, g.n_rows / 32)));
+    const int64_t b = std::min<int64_t>((int64_t)sms * 8, most / 256 + 1);
+    k_plan_setup<<<(unsigned)b, 256, 0, st>>>(g, p, uvw, freq, chan_map, delta_l, delta_m);
     AV_LAUNCH_CHECK();
   }
-  int sms = sm_count();
   // one warp per (baseline, 32 time steps) unit, 8 warps per block
   int64_t blocks = (g.nb * ((g.nt + 31) / 32) + 7) / 8;
   if (blocks > (int64_t)sms * 16) blocks = (int64_t)sms * 16;
@@ -684,17 +722,13 @@ int plan_build(const PlanGeom &g, Plan &p, const double *uvw, const double *freq
                                                   p.exc_count, p.exc_rows, drop_wt, drop_npol);
     AV_LAUNCH_CHECK();
   }
-  int rc = scan_counts(p.cursor, p.offs, nk + 1, p.scan_tmp, st);
+  int rc = scan_counts(g, p, nk + 1, st);
   if (rc) return rc;
   if (g.n_rows > 0) {
     k_plan_scatter<<<(unsigned)blocks, 256, 0, st>>>(g, p.walk_key, (const uint2 *)p.walk_rec,
                                                     p.cursor, (uint2 *)p.recs, p.exc_mark);
     AV_LAUNCH_CHECK();
   }
-  int64_t nt = g.n_tiles() + 1;
-  k_tile_starts<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(p.offs, g.n_tiles(), g.kpt,
-                                                              p.tile_start, p.counters);
-  AV_LAUNCH_CHECK();
   return AV_OK;
 }
 

@@ -14,7 +14,7 @@
 // scatter (warp-aggregated atomic cursors).  Order inside a key is the
 // arrival order of the atomics.  Samples that are skipped (off the grid, NaN
 // uvw, channel outside the image) go to one extra key, n_keys, after all
-// tiles: offs[n_keys] counts the usable records and the rest of recs[] lists
+// tiles: *n_rec counts the usable records and the rest of recs[] lists
 // the skipped rows (a store-mode degrid writes zeros there).
 //
 // A shared plan (convention 2) serves the gridder and the degridder at once:
@@ -128,7 +128,7 @@ inline void plan_geometry(PlanGeom &g, int64_t nt, int64_t nb, int64_t nchan,
 
 inline size_t plan_workspace_bytes(const PlanGeom &g) {
   size_t b = 0;
-  b += Workspace::need(sizeof(uint32_t) * (g.n_keys() + 2));  // offsets
+  b += Workspace::need(sizeof(uint32_t) * 4);                 // usable records
   b += Workspace::need(sizeof(uint32_t) * (g.n_keys() + 2));  // cursors
   b += Workspace::need(sizeof(uint32_t) * (g.n_tiles() + 1)); // tile starts
   b += Workspace::need(sizeof(Rec) * (g.n_rows > 0 ? g.n_rows : 1));
@@ -156,9 +156,9 @@ inline size_t plan_workspace_bytes(const PlanGeom &g) {
 }
 
 struct Plan {
-  uint32_t *offs;      // n_keys + 2: start of each key (exclusive scan); the
-                       // last key (n_keys) holds the skipped samples
-  uint32_t *cursor;    // n_keys + 2
+  uint32_t *n_rec;     // [0]: usable records
+  uint32_t *cursor;    // n_keys + 2: counts, then starts, and after the scatter pass
+                       // the end of each key (the last one holds the skipped samples)
   uint32_t *tile_start;// n_tiles + 1
   Rec *recs;           // n_rows (only the first n_rec are used)
   double *scale;       // 2 * nchan: per-channel uv scale (gridder convention)
@@ -258,7 +258,7 @@ __device__ __forceinline__ bool sample_pos_degrid(double um, double vm, double f
 
 // Host: enqueue the plan build for uvw / freq / chan_map (plane per channel;
 // entries outside [0, n_planes) drop the channel).  Nothing is synchronised:
-// the record count stays on the device in offs[n_keys] (and a shared plan's
+// the record count stays on the device in n_rec (and a shared plan's
 // exception count in exc_count[0]).  A shared plan (g.convention == 2) needs
 // the degridder's scale / offset / bounds extents in g as well as the
 // gridder's cell size (delta_l, delta_m).
