@@ -20,7 +20,8 @@ _DT = {torch.float32: AV_F32, torch.float64: AV_F64, torch.complex64: AV_C64,
 
 
 def require_gpu():
-    if not torch.cuda.is_available():
+    # an initialised CUDA context answers without asking the driver again
+    if not (torch.cuda.is_initialized() or torch.cuda.is_available()):
         raise RuntimeError("astroviper_b200 needs a CUDA device (B200, sm_100a); none is visible")
     lib()
 
@@ -31,7 +32,9 @@ def device():
 
 
 def stream_ptr():
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream (without a Stream object: every kernel
+    call asks for it)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def dcode(t):
@@ -65,6 +68,39 @@ def on_device(x, dtype=None):
     else:
         t = torch.as_tensor(x, dtype=dtype, device=dev)
     return t.contiguous()
+
+
+_NP_OF = {torch.float64: np.float64, torch.int32: np.int32}
+
+
+def upload(*items):
+    """Contiguous CUDA tensors of (array or tensor, dtype) pairs, dtype
+    float64 or int32.  The host arrays among them (frequencies, channel and
+    polarisation maps: a few hundred bytes each) go up together, in one
+    asynchronous copy from page-locked memory; one copy each from pageable
+    memory made the host wait for every one of them."""
+    out = [None] * len(items)
+    pack, size = [], 0
+    for i, (x, dt) in enumerate(items):
+        if isinstance(x, torch.Tensor):
+            out[i] = on_device(x, dt)
+        else:
+            a = np.ascontiguousarray(np.asarray(x), dtype=_NP_OF[dt])
+            pack.append((i, a, size))
+            size += (a.nbytes + 15) & ~15
+    if size == 0:
+        for i, a, _ in pack:
+            out[i] = torch.empty(a.shape, dtype=items[i][1], device=device())
+        return out
+    dev = device()
+    host = torch.empty(size, dtype=torch.uint8, pin_memory=True)
+    view = host.numpy()
+    for i, a, at in pack:
+        view[at:at + a.nbytes] = a.reshape(-1).view(np.uint8)
+    buf = host.to(dev, non_blocking=True)
+    for i, a, at in pack:
+        out[i] = buf[at:at + a.nbytes].view(items[i][1]).view(a.shape)
+    return out
 
 
 def on_device_flag(flag):
@@ -164,10 +200,8 @@ def grid(vis, weight, uvw, freq, chan_map, pol_map, cgk, n_uv, delta_lm, support
     nt, nb = int(uvw.shape[0]), int(uvw.shape[1])
     nchan, npol = int(weight.shape[2]), int(weight.shape[3])
     uvw = on_device(uvw, torch.float64)
-    freq = on_device(freq, torch.float64)
-    cm = on_device(chan_map, torch.int32)
-    pm = on_device(pol_map, torch.int32)
-    cgk = on_device(cgk, torch.float64)
+    freq, cm, pm, cgk = upload((freq, torch.float64), (chan_map, torch.int32),
+                               (pol_map, torch.int32), (cgk, torch.float64))
     fp64 = not grid_tiled_ok(precision, do_imaging_weight, support, oversampling, npol,
                              n_img_pol)
     if grid_out is None:
@@ -234,10 +268,8 @@ def degrid(grid_t, uvw, freq, scale, offset, chanmap, polmap, cgk, support, samp
     if values is not None:
         nvchan, nvpol = int(values.shape[2]), int(values.shape[3])
     uvw = on_device(uvw, torch.float64)
-    freq = on_device(freq, torch.float64)
-    cm = on_device(chanmap, torch.int32)
-    pm = on_device(polmap, torch.int32)
-    cgk = on_device(cgk, torch.float64)
+    freq, cm, pm, cgk = upload((freq, torch.float64), (chanmap, torch.int32),
+                               (polmap, torch.int32), (cgk, torch.float64))
     fl = on_device_flag(flag)
     dph = None if dphase is None else on_device(dphase, torch.float64)
     g_nchan, g_npol, g_n2, g_n3 = (int(s) for s in g.shape)
@@ -665,9 +697,21 @@ def pol_transform(x, matrix, pol_axis, out_dtype):
     return out
 
 
+def argmax_value(x, mode):
+    """The value of argmax(x, mode) as a float64 device tensor of one element;
+    nothing is waited for."""
+    return _argmax(x, mode)[1][:1]
+
+
 def argmax(x, mode):
     """(index, value) of np.argmax(np.abs(x)) (mode 0) / np.argmax(x) (mode 1)
     over the flattened x; value is x at that index.  Synchronises."""
+    idx, res = _argmax(x, mode)
+    both = torch.cat([idx.view(torch.float64), res[:1]]).cpu()
+    return int(both[:1].view(torch.int64).item()), float(both[1].item())
+
+
+def _argmax(x, mode):
     t = on_device(x)
     if t.dtype not in (torch.float32, torch.float64):
         t = t.to(torch.float64)
@@ -677,7 +721,7 @@ def argmax(x, mode):
     _buf, wptr, wbytes = workspace(lib().av_argmax_workspace_size(n))
     check(lib().av_argmax(p(t), dcode(t), n, int(mode), p(idx), p(res), wptr, wbytes,
                           stream_ptr()), "av_argmax")
-    return int(idx.item()), float(res[0].item())
+    return idx, res
 
 
 def psf_sidelobe(psf, window=(41, 41), threshold=0.35):
@@ -763,10 +807,9 @@ def mosaic_grid(grid, sum_weight, do_psf, vis, weight, uvw, freq, chan_map, pol_
     nt, nb, nchan, npol = (int(s) for s in w.shape)
     v = None if (do_psf or aperture) else on_device(vis, torch.complex128)
     uvw_d = on_device(uvw, torch.float64)
-    freq_d = on_device(freq, torch.float64)
-    maps = [on_device(np.asarray(m), torch.int32) for m in
-            (chan_map, pol_map, cfb_map, cfc_map, cfp_map)]
-    sup = on_device(np.asarray(support), torch.int32)
+    freq_d, sup, *maps = upload((freq, torch.float64), (np.asarray(support), torch.int32),
+                                *[(np.asarray(m), torch.int32) for m in
+                                  (chan_map, pol_map, cfb_map, cfc_map, cfp_map)])
     n_cfb, n_cfc, n_cfp, cu, cv = (int(s) for s in cf.shape)
     os_u, os_v = (int(oversampling[0]), int(oversampling[1])) if np.ndim(oversampling) else \
         (int(oversampling), int(oversampling))

@@ -121,13 +121,14 @@ def _masksum(image, dv):
 def _peak_residual(plane, mask=None):
     """image_peak_residual of one plane (image_statistics.py:40-88,
     per_plane_stats=False): the value at the largest |x|, masked pixels out
-    (NaN, as xarray's where leaves them) when a mask is given."""
+    (NaN, as xarray's where leaves them) when a mask is given; one element on
+    the device."""
     t = K.on_device(plane)
     if mask is not None:
         m = K.on_device(mask)
         t = torch.where(m.to(torch.bool), t.to(torch.float64),
                         torch.full((), float("nan"), dtype=torch.float64, device=t.device))
-    return K.argmax(t, 0)[1]
+    return K.argmax_value(t, 0)
 
 
 def _device_cube(values):
@@ -207,11 +208,14 @@ def deconvolve(dirty_image_xds, psf_xds, model_xds=None, algorithm: str = "hogbo
                     progress=False)
                 model_out[tt, nn, pp] = model_arr
                 resid_out[tt, nn, pp] = resid_arr
-                flux = float(K.plane_sum(model_arr).item())
-                if model_arr.dtype == torch.float32:
-                    flux = float(np.float32(flux))  # np.sum of a float32 plane
                 peakres = _peak_residual(resid_out[tt, nn, pp], mk)
                 peakres_nomask = peakres if mk is None else _peak_residual(resid_out[tt, nn, pp])
+                # the plane's statistics in one read
+                (start_peakres, start_peakres_nomask, peakres, peakres_nomask,
+                 flux) = torch.cat([start_peakres, start_peakres_nomask, peakres, peakres_nomask,
+                                    K.plane_sum(model_arr).reshape(1)]).tolist()
+                if model_arr.dtype == torch.float32:
+                    flux = float(np.float32(flux))  # np.sum of a float32 plane
                 rd.add({
                     "niter": deconv_params.get("niter", None),
                     "threshold": deconv_params.get("threshold", None),

@@ -339,7 +339,8 @@ def run_imaging_loop(ms4, params: Dict[str, Any], initial_model: Optional[np.nda
             dirty_img["RESIDUAL"].values[0].copy_(dirty_stokes)
         if major_cycle == 1:
             temp = ReturnDict()
-            temp.add({"peakres": _abs_max(dirty_stokes), "peakres_nomask": _abs_max(dirty_stokes),
+            peak = _abs_max(dirty_stokes)
+            temp.add({"peakres": peak, "peakres_nomask": peak,
                       "masksum": ny * nx, "iter_done": 0, "max_psf_sidelobe": 0.2,
                       "loop_gain": gain}, time=0, pol=0, chan=0)
             cycle_niter, cyclethresh = controller.calculate_cycle_controls(temp)

@@ -11,6 +11,7 @@ defines them, since they fix the scale of every Stokes image it produces.
 numpy input gives numpy output; torch tensors stay on the device.  xarray
 DataArrays are accepted when xarray is installed.
 """
+import sys
 from typing import List, Optional
 
 import numpy as np
@@ -53,11 +54,9 @@ _STOKES_INDEX = {"I": 0, "Q": 1, "U": 2, "V": 3}
 
 
 def _xr_dataarray():
-    try:
-        import xarray
-        return xarray.DataArray
-    except Exception:
-        return None
+    """xarray.DataArray where a caller has imported xarray (its data could not
+    be a DataArray otherwise; a failing import searches the path every time)."""
+    return getattr(sys.modules.get("xarray"), "DataArray", None)
 
 
 def _table(corr_type, transformation_matrix, linear, circular):
