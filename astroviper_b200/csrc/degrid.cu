@@ -484,7 +484,9 @@ __global__ void __launch_bounds__(DT_THREADS) k_degrid_tiled(TiledDegridArgs a) 
   // persistent: chunks of records from a.sched[0] until none are left
   for (;;) {
   __syncthreads();  // tables built; the previous chunk is done with sub and s_chunk
-  if (threadIdx.x == 0) s_chunk = (int)atomicAdd(&a.sched[0], 1u);
+  if (threadIdx.x == 0)
+    s_chunk = chunk_in_turn(atomicAdd(&a.sched[0], 1u), (uint32_t)n_chunks,
+                              (uint32_t)(a.n_tiles / (a.ntu * a.ntv)));
   __syncthreads();
   const int64_t ch = s_chunk;
   if (ch >= n_chunks) break;
@@ -754,7 +756,9 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_degrid_tc(TiledDegridArgs a) 
 
   for (;;) {
     __syncthreads();  // tables built; the previous chunk is done with sub and s_chunk
-    if (threadIdx.x == 0) s_chunk = (int)atomicAdd(&a.sched[0], 1u);
+    if (threadIdx.x == 0)
+      s_chunk = chunk_in_turn(atomicAdd(&a.sched[0], 1u), (uint32_t)n_chunks,
+                              (uint32_t)(a.n_tiles / (a.ntu * a.ntv)));
     __syncthreads();
     const int64_t ch = s_chunk;
     if (ch >= n_chunks) break;
@@ -1187,7 +1191,9 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_degrid_umma(TiledDegridArgs a
 
   for (;;) {
     __syncthreads();
-    if (tid == 0) s_chunk = (int)atomicAdd(&a.sched[0], 1u);
+    if (tid == 0)
+      s_chunk = chunk_in_turn(atomicAdd(&a.sched[0], 1u), (uint32_t)n_chunks,
+                              (uint32_t)(a.n_tiles / (a.ntu * a.ntv)));
     __syncthreads();
     const int64_t ch = s_chunk;
     if (ch >= n_chunks) break;
@@ -1616,8 +1622,21 @@ static int launch_degrid_sorted(const SortedDegridArgs &a, int64_t rows, cudaStr
   return AV_OK;
 }
 
+// Chunks of records the persistent CTAs take one at a time: per_sm for each
+// SM, of 1024 records at least, so that a chunk's tile loads stay small
+// against its samples; sets a.chunk and returns their number.
+// AV_TUNE_DEGRID_CHUNKS_PER_SM (16) is k_degrid_tc's (33M samples: 8 830 us,
+// 16 768, 24 791); k_degrid_tiled's CTAs take half as many, twice as long
+// (4.2M samples of one polarisation: 16 97 us, 8 89; 2.06M of two: 90, 82).
+static int64_t degrid_chunking(TiledDegridArgs &a, int64_t per_sm) {
+  const int64_t parts = (int64_t)sm_count() * per_sm;
+  a.chunk = std::max<int64_t>(1024, (a.n_rows + parts - 1) / parts);
+  return (a.n_rows + a.chunk - 1) / a.chunk;
+}
+
 template <int S>
-static int launch_degrid_tc(const TiledDegridArgs &a, int64_t nblocks, cudaStream_t st) {
+static int launch_degrid_tc(TiledDegridArgs a, cudaStream_t st) {
+  int64_t nblocks = degrid_chunking(a, tune_value(AV_TUNE_DEGRID_CHUNKS_PER_SM));
   size_t smem = TCSmem<S>::total;
   static int resident[64] = {0};
   int dev = 0;
@@ -1642,7 +1661,8 @@ static int launch_degrid_tc(const TiledDegridArgs &a, int64_t nblocks, cudaStrea
 }
 
 template <int S>
-static int launch_degrid_umma(const TiledDegridArgs &a, int64_t nblocks, cudaStream_t st) {
+static int launch_degrid_umma(TiledDegridArgs a, cudaStream_t st) {
+  int64_t nblocks = degrid_chunking(a, tune_value(AV_TUNE_DEGRID_CHUNKS_PER_SM));
   const size_t smem = UMSmem<S>::total;
   static bool attr[64] = {false};
   int dev = 0;
@@ -1666,7 +1686,9 @@ static int launch_degrid_umma(const TiledDegridArgs &a, int64_t nblocks, cudaStr
 }
 
 template <int S, int NPG, bool STORE>
-static int launch_degrid_tiled_as(const TiledDegridArgs &a, int64_t nblocks, cudaStream_t st) {
+static int launch_degrid_tiled_as(TiledDegridArgs a, cudaStream_t st) {
+  const int64_t per_sm_chunks = tune_value(AV_TUNE_DEGRID_CHUNKS_PER_SM) / 2;
+  int64_t nblocks = degrid_chunking(a, std::max<int64_t>(1, per_sm_chunks));
   // persistent CTAs: at most as many as are resident at once
   size_t smem = DSmem<S, NPG>::total;
   static int resident[64] = {0};
@@ -1692,40 +1714,39 @@ static int launch_degrid_tiled_as(const TiledDegridArgs &a, int64_t nblocks, cud
 }
 
 template <int S, int NPG>
-static int launch_degrid_tiled(const TiledDegridArgs &a, int64_t nblocks, cudaStream_t st) {
-  return a.store ? launch_degrid_tiled_as<S, NPG, true>(a, nblocks, st)
-                 : launch_degrid_tiled_as<S, NPG, false>(a, nblocks, st);
+static int launch_degrid_tiled(const TiledDegridArgs &a, cudaStream_t st) {
+  return a.store ? launch_degrid_tiled_as<S, NPG, true>(a, st)
+                 : launch_degrid_tiled_as<S, NPG, false>(a, st);
 }
 
 // The TF32 tensor-core kernel for the fast store path with 4 grid
 // polarisations as AV_TUNE_DEGRID_LANES says (automatically for every support
 // it covers, 3-8, where it is the faster), the FP32 kernel otherwise.
 template <int S>
-static int degrid_dispatch_npg(const TiledDegridArgs &a, int npg, int64_t nb, cudaStream_t st) {
-  if (npg == 1) return launch_degrid_tiled<S, 1>(a, nb, st);
-  if (npg == 2) return launch_degrid_tiled<S, 2>(a, nb, st);
+static int degrid_dispatch_npg(const TiledDegridArgs &a, int npg, cudaStream_t st) {
+  if (npg == 1) return launch_degrid_tiled<S, 1>(a, st);
+  if (npg == 2) return launch_degrid_tiled<S, 2>(a, st);
   if constexpr (S <= 8) {
     const int64_t lanes = tune_value(AV_TUNE_DEGRID_LANES);
     if (a.fast_out && a.d.g_npol == 4 && lanes == AV_DEGRID_LANES_TC05)
-      return launch_degrid_umma<S>(a, nb, st);
+      return launch_degrid_umma<S>(a, st);
     const bool tf32 = lanes == AV_DEGRID_LANES_TF32 || lanes == AV_DEGRID_LANES_AUTO;
     // the TF32 kernel keeps a shared plan's marks in the staged rows' top bit
     if (a.fast_out && a.d.g_npol == 4 && tf32 && a.n_rows < (int64_t)REC_DEGRID_EXC)
-      return launch_degrid_tc<S>(a, nb, st);
+      return launch_degrid_tc<S>(a, st);
   }
-  return launch_degrid_tiled<S, 4>(a, nb, st);
+  return launch_degrid_tiled<S, 4>(a, st);
 }
 
-static int degrid_dispatch(const TiledDegridArgs &a, int support, int npg, int64_t nb,
-                           cudaStream_t st) {
+static int degrid_dispatch(const TiledDegridArgs &a, int support, int npg, cudaStream_t st) {
   switch (support) {
-    case 3: return degrid_dispatch_npg<3>(a, npg, nb, st);
-    case 4: return degrid_dispatch_npg<4>(a, npg, nb, st);
-    case 5: return degrid_dispatch_npg<5>(a, npg, nb, st);
-    case 6: return degrid_dispatch_npg<6>(a, npg, nb, st);
-    case 7: return degrid_dispatch_npg<7>(a, npg, nb, st);
-    case 8: return degrid_dispatch_npg<8>(a, npg, nb, st);
-    case 9: return degrid_dispatch_npg<9>(a, npg, nb, st);
+    case 3: return degrid_dispatch_npg<3>(a, npg, st);
+    case 4: return degrid_dispatch_npg<4>(a, npg, st);
+    case 5: return degrid_dispatch_npg<5>(a, npg, st);
+    case 6: return degrid_dispatch_npg<6>(a, npg, st);
+    case 7: return degrid_dispatch_npg<7>(a, npg, st);
+    case 8: return degrid_dispatch_npg<8>(a, npg, st);
+    case 9: return degrid_dispatch_npg<9>(a, npg, st);
   }
   set_error("av_degrid_tiled: support %d not in [3, 9]", support);
   return AV_ERR_UNSUPPORTED;
@@ -1907,12 +1928,8 @@ int av_degrid_tiled_execute(const double *dphase, void *values, int values_dtype
   a.n_tiles = g.n_tiles();
   a.ntu = g.ntu;
   a.ntv = g.ntv;
-  int sms = sm_count();
-  const int64_t per_sm = tune_value(AV_TUNE_DEGRID_CHUNKS_PER_SM);
-  int64_t chunk = (rows + (int64_t)sms * per_sm - 1) / ((int64_t)sms * per_sm);
-  if (chunk < 1024) chunk = 1024;
-  a.chunk = chunk;
   a.d = d;
+  const int sms = sm_count();
   a.cgk_len = sampling * (support / 2 + 1);
   a.sched = p.counters + 2;
   a.accumulate = accumulate ? 1 : 0;
@@ -1924,7 +1941,7 @@ int av_degrid_tiled_execute(const double *dphase, void *values, int values_dtype
   a.wide_values = (((uintptr_t)values) & 15) == 0;
   a.wide_flags = flag != nullptr && (((uintptr_t)flag) & (uintptr_t)(nvpol - 1)) == 0;
   int npg = g_npol <= 1 ? 1 : (g_npol <= 2 ? 2 : 4);
-  rc = degrid_dispatch(a, support, npg, (rows + chunk - 1) / chunk, as_stream(stream));
+  rc = degrid_dispatch(a, support, npg, as_stream(stream));
   if (rc) return rc;
   // a shared plan's exceptions (none listed in a degridder plan: the kernel
   // reads a zero count and returns)

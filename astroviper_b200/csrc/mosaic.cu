@@ -350,7 +350,9 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mosaic_tiled(MosaicTiledArgs 
   }
   for (;;) {
     __syncthreads();  // sub-grid clear; previous s_chunk consumed
-    if (threadIdx.x == 0) s_chunk = (int)atomicAdd(&t.sched[0], 1u);
+    if (threadIdx.x == 0)
+      s_chunk = chunk_in_turn(atomicAdd(&t.sched[0], 1u), (uint32_t)n_chunks,
+                              (uint32_t)(t.n_tiles / (t.ntu * t.ntv)));
     __syncthreads();
     const int64_t ch = s_chunk;
     if (ch >= n_chunks) break;
@@ -505,7 +507,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mosaic_tiled(MosaicTiledArgs 
 // Cells past the window hold zero taps, so only an infinite value, whose
 // product with them would be NaN, needs the window's true extent; such
 // samples (rare) are masked tap by tap.
-// 1.03M samples x 2 polarisations, supports 5-7: 1315 us before, 257 us now (and 70 us of plan).
+// 1.03M samples x 2 polarisations, supports 5-7: 1315 us before, 207 us now (and 45 us of plan).
 constexpr int MR_MAX_S = 11;
 constexpr int MR_THREADS = 256;
 constexpr int MR_WARPS = MR_THREADS / 32;
@@ -640,8 +642,9 @@ __global__ void __launch_bounds__(MR_THREADS, CPL *NPOL <= 4 ? 2 : 1)
   const MosaicTiledArgs &t = q.t;
   const MosaicArgs &a = t.m;
   constexpr int NF = MULTI ? NPOL : 1;  // tap rows per sample
-  // samples whose taps are loaded together: up to 8 loads in flight per lane
-  constexpr int AHEAD = NF * CPL <= 2 ? 4 : (NF * CPL <= 4 ? 2 : 1);
+  // samples whose taps are loaded together, up to 8 loads in flight per lane (2
+  // at a time take 225 us of the 1.03M samples, 4 256 us for their registers)
+  constexpr int AHEAD = NF * CPL <= 4 ? 2 : 1;
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int S = t.S, S2 = S * S, npg = (int)a.n_img_pol;
@@ -676,7 +679,9 @@ __global__ void __launch_bounds__(MR_THREADS, CPL *NPOL <= 4 ? 2 : 1)
   const int64_t n_chunks = ((int64_t)n_rec + t.chunk - 1) / t.chunk;
   for (;;) {
     __syncthreads();  // sub-grid clear; previous s_chunk consumed
-    if (threadIdx.x == 0) s_chunk = (int)atomicAdd(&t.sched[0], 1u);
+    if (threadIdx.x == 0)
+      s_chunk = chunk_in_turn(atomicAdd(&t.sched[0], 1u), (uint32_t)n_chunks,
+                              (uint32_t)(t.n_tiles / (t.ntu * t.ntv)));
     __syncthreads();
     const int64_t ch = s_chunk;
     if (ch >= n_chunks) break;

@@ -62,7 +62,7 @@ unsigned long long av_launch_count(void);
  * process-wide knobs read when a kernel is launched, set by the autotuner
  * (astroviper_b200.autotune) or by hand.
  *   AV_TUNE_GRID_CHUNKS_PER_SM   record chunks per SM handed out by the
- *                                persistent tiled gridder (default 16)
+ *                                persistent tiled gridder (default 8)
  *   AV_TUNE_DEGRID_CHUNKS_PER_SM record chunks per SM handed out by the
  *                                persistent tiled degridder (default 16)
  *   AV_TUNE_GRID_LANES           how the tiled gridder sums a run of samples:
