@@ -134,15 +134,18 @@ class Gridder:
         """Build the gridding and the degridding plan (for a grid of g_nchan
         channels, default n_img_chan).  When the degridder's channel map
         int(i / nchan * g_nchan) equals the gridder's (continuum and cube
-        images), one shared plan serves both (av_tiled_plan_shared): the two
-        conventions differ only in their rounding, and the rare samples where
-        that matters are degridded apart in FP64.  Otherwise the two plans
+        images) and both image sizes are even, one shared plan serves both
+        (av_tiled_plan_shared): the two conventions then differ only in their
+        rounding, and the rare samples where that matters are degridded apart
+        in FP64.  (The gridder's centre is cell n // 2, the degridder's n / 2:
+        half a cell apart for an odd size.)  Otherwise the two plans
         are built concurrently on two streams: both depend only on uvw, the
         frequencies and the geometry, and neither fills the GPU alone.  Later
         calls on the current stream see the plans."""
         key = int(self.n_img_chan if g_nchan is None else g_nchan)
         dmap = (np.arange(self.nchan) / self.nchan * key).astype(int)
         if (self.shared_plan and key == self.n_img_chan
+                and self.nx % 2 == 0 and self.ny % 2 == 0
                 and np.array_equal(dmap, self._cm_host)):
             need = lib().av_grid_tiled_workspace_size(self.nt, self.nb, self.nchan, self.nx,
                                                       self.ny, self.n_img_chan, self.support)
