@@ -1213,9 +1213,9 @@ static int launch_grid_mma(const TiledGridArgs &a, int64_t nblocks, cudaStream_t
 // 5-8: with smaller footprints most of the 8 x 8 tile is padding and the row
 // lanes are faster); k_grid_tiled otherwise (support 9).  The degridder's
 // adjoint follows the same rule: 4.16M samples of one polarisation, support 7,
-// take 145 us against 210 us of the row lanes.  Double-precision inputs take
+// take 126 us (145 in record order, the row lanes 210).  Double-precision inputs take
 // k_grid_mma for every support it covers, whatever the knob says: 806k
-// samples of 2 polarisations take 78 us, and 31 us of plan, against 2620 us of
+// samples of 2 polarisations take 65 us, and 31 us of plan, against 2620 us of
 // k_grid_plain, whose 98 global FP64 atomics per correlation bound it.
 template <int S, int NPOL>
 static int launch_grid_tiled(const TiledGridArgs &a, int64_t nblocks, cudaStream_t st) {
