@@ -117,19 +117,31 @@ __global__ void k_ishift_in(const IT *in, CT *buf, int64_t nplanes, int64_t nx, 
 // thread evaluates the grid correction's factor of its column once and the
 // block the factors of its rows once: an evaluation per pixel, a long chain
 // of FP64 operations and divides, had made the epilogue of four 2048^2 images
-// 548 us (now 85).  IMG_UNROLL rows in flight per thread.  16 rows to a block
-// give a 1024^2 image enough blocks (prologue and epilogue 20 us; 30 with
-// 32 rows), 32 would take four 2048^2 images from 85 to 78.
+// 548 us (85 with the factors per row and column, 61 now).  IMG_UNROLL rows in
+// flight per thread: 8 take the epilogue there from 68 to 61 us and the gather
+// from 65 to 62 against 4, 2 79 us.  16 rows to a block give a 1024^2 image
+// enough blocks (prologue and epilogue 20 us; 30 with 32 rows).
 // The real transforms themselves halve what the complex ones moved: the
-// gather 95 -> 65 us and cuFFT 289 -> 175 us for four 2048^2 planes, whole
-// images 932 -> 325 us.  Batches of planes small enough to stay in L2 between
+// gather 95 -> 62 us and cuFFT 289 -> 175 us for four 2048^2 planes, whole
+// images 932 -> 302 us.  Batches of planes small enough to stay in L2 between
 // the passes gained nothing (374 us: cuFFT is bound by its FP64 work there).
-constexpr int IMG_COLS = 128, IMG_ROWS = 16, IMG_UNROLL = 4;
+constexpr int IMG_COLS = 128, IMG_ROWS = 16, IMG_UNROLL = 8;
 
 static dim3 img_grid(int64_t nplanes, int64_t rows, int64_t cols) {
   return dim3((unsigned)((cols + IMG_COLS - 1) / IMG_COLS),
               (unsigned)std::min<int64_t>((rows + IMG_ROWS - 1) / IMG_ROWS, 65535),
               (unsigned)std::min<int64_t>(nplanes, 65535));
+}
+
+// For the passes with the grid correction: two planes to a block where that
+// leaves 16 blocks per SM, so a factor serves twice the pixels (four 2048^2
+// images 68 -> 61 us).
+static dim3 pixel_grid(int64_t nplanes, int64_t nx, int64_t ny) {
+  dim3 g = img_grid(nplanes, nx, ny);
+  const int64_t pairs = (nplanes + 1) / 2;
+  if (pairs <= 65535 && (int64_t)g.x * g.y * pairs >= (int64_t)sm_count() * 16)
+    g.z = (unsigned)pairs;
+  return g;
 }
 
 // i + s for 0 <= i < n, 0 <= s <= n, modulo n.
@@ -157,13 +169,24 @@ __device__ __forceinline__ double quotient(double v, double d, double r) {
   return fma(fma(-q, d, v), r, q);
 }
 
-// Calls f(plane, row, column, ...) for every pixel of this block's share,
-// IMG_UNROLL rows at a time: f.load first, then f.store with the grid
-// correction's factors and their reciprocals (1 without apply_corr).
+// v / d for r = 1 / d rounded: as above without the Newton step.
+__device__ __forceinline__ double quotient_by(double v, double d, double r) {
+  const double q = v * r;
+  const double m = fabs(q);
+  if (!(m > 1e-250 && m < 1e250)) return v / d;
+  return fma(fma(-q, d, v), r, q);
+}
+
+// Carries every pixel of this block's share from f.in to f.out, IMG_UNROLL
+// rows at a time, with the grid correction's factors and their reciprocals (1
+// without apply_corr).  The rows' wrapped offsets are worked out once for the
+// block's planes: 64-bit index arithmetic per pixel had made the pass issue
+// bound.
 template <typename F>
 __device__ __forceinline__ void for_pixels(int64_t nplanes, int64_t nx, int64_t ny,
                                            int apply_corr, F f) {
   __shared__ double2 s_gx[IMG_ROWS];
+  __shared__ int64_t s_in[IMG_ROWS], s_out[IMG_ROWS];
   const int64_t j = blockIdx.x * (int64_t)IMG_COLS + threadIdx.x;
   double2 gy = make_double2(1.0, 1.0);
   if (apply_corr && j < ny) {
@@ -174,22 +197,32 @@ __device__ __forceinline__ void for_pixels(int64_t nplanes, int64_t nx, int64_t 
        i0 += gridDim.y * (int64_t)IMG_ROWS) {
     __syncthreads();
     if (threadIdx.x < IMG_ROWS && i0 + threadIdx.x < nx) {
-      const double g = apply_corr ? corr_factor(i0 + threadIdx.x, nx) : 1.0;
+      const int64_t i = i0 + threadIdx.x;
+      const double g = apply_corr ? corr_factor(i, nx) : 1.0;
       s_gx[threadIdx.x] = make_double2(g, 1.0 / g);
+      s_in[threadIdx.x] = f.row_in(i);
+      s_out[threadIdx.x] = f.row_out(i);
     }
     __syncthreads();
     if (j >= ny) continue;
     const int rows = (int)std::min<int64_t>(IMG_ROWS, nx - i0);
     for (int64_t p = blockIdx.z; p < nplanes; p += gridDim.z) {
       const double sw = f.sumw ? f.sumw[p] : 1.0, rsw = 1.0 / sw;
+      const auto *in = f.in + p * f.plane_in() + f.col_in(j);
+      auto *out = f.out + p * f.plane_out() + f.col_out(j);
       for (int r = 0; r < rows; r += IMG_UNROLL) {
         double v[IMG_UNROLL];
 #pragma unroll
         for (int k = 0; k < IMG_UNROLL; ++k)
-          if (r + k < rows) v[k] = f.load(p, i0 + r + k, j);
+          if (r + k < rows) v[k] = (double)in[s_in[r + k]];
 #pragma unroll
         for (int k = 0; k < IMG_UNROLL; ++k)
-          if (r + k < rows) f.store(p, i0 + r + k, j, v[k], s_gx[r + k], gy, sw, rsw);
+          if (r + k < rows) {
+            const double2 gx = s_gx[r + k];
+            if (apply_corr) v[k] = quotient(v[k], gx.x * gy.x, gx.y * gy.y);
+            if (f.sumw) v[k] = quotient_by(v[k], sw, rsw);
+            f.store(out + s_out[r + k], v[k]);
+          }
       }
     }
   }
@@ -235,21 +268,20 @@ __global__ void __launch_bounds__(IMG_COLS) k_herm_in(const IT *grid, double2 *b
 // img[i, j] = t[(i + nx - nx/2) % nx, (j + ny - ny/2) % ny] / (gx gy) / sumw.
 template <typename OT>
 struct ImageEpilogue {
-  const double *buf;
-  OT *img;
+  const double *in;
+  OT *out;
   const double *sumw;
   int64_t nx, ny;
   int apply_corr;
-  __device__ __forceinline__ double load(int64_t p, int64_t i, int64_t j) const {
-    return buf[(p * nx + wrap(i, nx - nx / 2, nx)) * (2 * half_cols(ny)) +
-               wrap(j, ny - ny / 2, ny)];
+  __device__ int64_t plane_in() const { return nx * 2 * half_cols(ny); }
+  __device__ int64_t plane_out() const { return nx * ny; }
+  __device__ int64_t row_in(int64_t i) const {
+    return wrap(i, nx - nx / 2, nx) * 2 * half_cols(ny);
   }
-  __device__ __forceinline__ void store(int64_t p, int64_t i, int64_t j, double v, double2 gx,
-                                        double2 gy, double sw, double rsw) const {
-    if (apply_corr) v = quotient(v, gx.x * gy.x, gx.y * gy.y);
-    if (sumw) v = quotient(v, sw, rsw);
-    __stcs(img + (p * nx + i) * ny + j, (OT)v);
-  }
+  __device__ int64_t row_out(int64_t i) const { return i * ny; }
+  __device__ int64_t col_in(int64_t j) const { return wrap(j, ny - ny / 2, ny); }
+  __device__ int64_t col_out(int64_t j) const { return j; }
+  __device__ void store(OT *at, double v) const { __stcs(at, (OT)v); }
 };
 
 template <typename OT>
@@ -262,20 +294,20 @@ __global__ void __launch_bounds__(IMG_COLS) k_image_epilogue(ImageEpilogue<OT> f
 // grid correction when asked.
 template <typename IT>
 struct ImagePrologue {
-  const IT *img;
-  double *buf;
+  const IT *in;
+  double *out;
   const double *sumw;  // none
   int64_t nx, ny;
   int apply_corr;
-  __device__ __forceinline__ double load(int64_t p, int64_t i, int64_t j) const {
-    return (double)img[(p * nx + i) * ny + j];
+  __device__ int64_t plane_in() const { return nx * ny; }
+  __device__ int64_t plane_out() const { return nx * 2 * half_cols(ny); }
+  __device__ int64_t row_in(int64_t i) const { return i * ny; }
+  __device__ int64_t row_out(int64_t i) const {
+    return wrap(i, nx - nx / 2, nx) * 2 * half_cols(ny);
   }
-  __device__ __forceinline__ void store(int64_t p, int64_t i, int64_t j, double v, double2 gx,
-                                        double2 gy, double, double) const {
-    if (apply_corr) v = quotient(v, gx.x * gy.x, gx.y * gy.y);
-    buf[(p * nx + wrap(i, nx - nx / 2, nx)) * (2 * half_cols(ny)) + wrap(j, ny - ny / 2, ny)] =
-        v;
-  }
+  __device__ int64_t col_in(int64_t j) const { return j; }
+  __device__ int64_t col_out(int64_t j) const { return wrap(j, ny - ny / 2, ny); }
+  __device__ void store(double *at, double v) const { *at = v; }
 };
 
 template <typename IT>
@@ -423,7 +455,8 @@ int av_grid_to_image(const void *grid, int grid_dtype, const double *sum_weight,
   double2 *buf = ws.take<double2>(bufb / sizeof(double2));
   void *work = ws.take<char>(workb > 0 ? workb : 1);
   cudaStream_t st = as_stream(stream);
-  const dim3 half = img_grid(nplanes, nx, half_cols(ny)), full = img_grid(nplanes, nx, ny);
+  const dim3 half = img_grid(nplanes, nx, half_cols(ny)),
+             full = pixel_grid(nplanes, nx, ny);
   if (grid_dtype == AV_C128)
     k_herm_in<double2><<<half, IMG_COLS, 0, st>>>((const double2 *)grid, buf, nplanes,
                                                   nx, ny);
@@ -468,13 +501,13 @@ int av_image_to_grid(const void *image, int image_dtype, void *grid, int grid_dt
   double2 *buf = ws.take<double2>(bufb / sizeof(double2));
   void *work = ws.take<char>(workb > 0 ? workb : 1);
   cudaStream_t st = as_stream(stream);
-  const dim3 full = img_grid(nplanes, nx, ny);
+  const dim3 full = img_grid(nplanes, nx, ny), pixels = pixel_grid(nplanes, nx, ny);
   if (image_dtype == AV_F64)
-    k_image_prologue<double><<<full, IMG_COLS, 0, st>>>(
+    k_image_prologue<double><<<pixels, IMG_COLS, 0, st>>>(
         ImagePrologue<double>{(const double *)image, (double *)buf, nullptr, nx, ny,
                               apply_corr}, nplanes);
   else
-    k_image_prologue<float><<<full, IMG_COLS, 0, st>>>(
+    k_image_prologue<float><<<pixels, IMG_COLS, 0, st>>>(
         ImagePrologue<float>{(const float *)image, (double *)buf, nullptr, nx, ny,
                              apply_corr}, nplanes);
   AV_LAUNCH_CHECK();

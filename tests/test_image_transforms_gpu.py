@@ -55,3 +55,18 @@ def test_real_image_forward_transform(nx, ny):
     assert _rel(fft_lm_to_uv(x.transpose(1, 2, 0), [0, 1]), ref.transpose(1, 2, 0)) <= 1e-14
     assert fft_lm_to_uv((10 * x).astype(np.int64), [1, 2]).dtype == np.complex128
     assert fft_lm_to_uv(x.astype(np.float32), [1, 2]).dtype == np.complex64
+
+
+@pytest.mark.parametrize("planes", [2367, 4735, 4737, 5000])
+def test_many_planes_take_a_block_for_two(planes):
+    """Around the number of blocks from which a block takes two planes (16 per
+    SM of 148), even and odd: each plane is the one of a call by itself."""
+    from astroviper_b200 import _kernels as K
+    rng = np.random.default_rng(planes)
+    g = rng.normal(size=(planes, 5, 4)) + 1j * rng.normal(size=(planes, 5, 4))
+    sw = rng.uniform(1.0, 2.0, planes)
+    got = K.grid_to_image(g, sw, apply_corr=False).cpu().numpy()
+    ref = _centred(g, np.fft.ifft2).real * 20 / sw[:, None, None]
+    assert np.abs(got - ref).max() <= 1e-14 * np.abs(ref).max()
+    one = K.grid_to_image(g[-1:], sw[-1:]).cpu().numpy()
+    assert np.abs(K.grid_to_image(g, sw).cpu().numpy()[-1:] - one).max() <= 1e-14 * np.abs(one).max()
