@@ -14,6 +14,8 @@
 //                     its function once.
 // av_cf_phase_product conv_kernel x phase_gradient[0] (mosaic_grid.py:384,
 //                     :56-58), elementwise without fused multiply-add.
+#include <math_constants.h>
+
 #include <algorithm>
 
 #include "plan.cuh"
@@ -497,16 +499,18 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mosaic_tiled(MosaicTiledArgs 
 //   - the taps of every function and kernel offset are first gathered into
 //     contiguous rows of S x S values (k_mosaic_taps), with the row's norm, so
 //     a sample's taps are one coalesced read where the oversampled function
-//     spreads them over a 32-byte sector each;
+//     spreads them over a 32-byte sector each; one more row, of zeros, is for
+//     samples without a value to add;
 //   - a warp's lanes stage 32 samples at once (weighted values, tap row, sum
 //     of weights), the next round's data in flight meanwhile;
 //   - lane l owns window cells l, l + 32, ... and keeps their sums for all
 //     polarisations while the samples stay in one cell: one tap load and 4
 //     NPOL DFMA per sample and owned cell, shared atomics only when the cell
 //     changes; four samples' taps are in flight whatever the runs.
-// Cells past the window hold zero taps, so only an infinite value, whose
-// product with them would be NaN, needs the window's true extent; such
-// samples (rare) are masked tap by tap.
+// Cells past the window hold zero taps and skipped values are zeros, so
+// products that the reference does not form are zeros too, unless the other
+// factor is not finite: a round with an infinite value or a row that holds a
+// tap that is not finite (both rare) goes tap by tap and value by value.
 // 1.03M samples x 2 polarisations, supports 5-7: 1315 us before, 207 us now (and 45 us of plan).
 constexpr int MR_MAX_S = 11;
 constexpr int MR_THREADS = 256;
@@ -515,9 +519,11 @@ constexpr int MR_ROUND = 32;  // samples a warp stages at once
 
 struct MosaicRunsArgs {
   MosaicTiledArgs t;
-  const double2 *taps;  // [function][u offset][v offset][S * S]
-  const double *norm;   // Re(norm) (PSF) or Re(norm^2) of each row
+  const double2 *taps;  // [function][u offset][v offset][S * S], then a row of zeros
+  const double2 *norm;  // per row: Re(norm) (PSF) or Re(norm^2); infinite when a
+                        // tap is not finite, else 0
   int first, n_off;     // kernel offsets first .. first + n_off - 1
+  int zero_row;
 };
 
 // Whether tap (iu, iv) counted from the window's corner is one of function
@@ -533,19 +539,21 @@ __device__ __forceinline__ bool mosaic_tap(const MosaicArgs &a, int64_t fidx, in
          iv >= -(sv / 2) && iv < sv - sv / 2 && fu >= 0 && fu < a.cu && fv >= 0 && fv < a.cv;
 }
 
-// One block per (function, u offset, v offset).
+// One block per (function, u offset, v offset), and one for the row of zeros.
 __global__ void __launch_bounds__(128) k_mosaic_taps(MosaicArgs a, int S, int first, int n_off,
-                                                     double2 *taps, double *norm) {
+                                                     double2 *taps, double2 *norm) {
   const int64_t row = blockIdx.x;
+  const bool zeros = row == gridDim.x - 1;
   const int ov = first + (int)(row % n_off), ou = first + (int)(row / n_off % n_off);
   const int64_t fidx = row / ((int64_t)n_off * n_off);
   double2 c = make_double2(0.0, 0.0);
   const int i = threadIdx.x;
   if (i < S * S) {
     int64_t at;
-    if (mosaic_tap(a, fidx, S, i / S, i % S, ou, ov, at)) c = a.cf[at];
+    if (!zeros && mosaic_tap(a, fidx, S, i / S, i % S, ou, ov, at)) c = a.cf[at];
     taps[row * (S * S) + i] = c;
   }
+  const int bad = __syncthreads_or(!isfinite(c.x) || !isfinite(c.y));
   __shared__ double2 sh[4];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -557,7 +565,8 @@ __global__ void __launch_bounds__(128) k_mosaic_taps(MosaicArgs a, int S, int fi
   if (i == 0) {
     const double x = (sh[0].x + sh[1].x) + (sh[2].x + sh[3].x);
     const double y = (sh[0].y + sh[1].y) + (sh[2].y + sh[3].y);
-    norm[row] = a.do_psf ? x : __dsub_rn(__dmul_rn(x, x), __dmul_rn(y, y));
+    norm[row] = make_double2(a.do_psf ? x : __dsub_rn(__dmul_rn(x, x), __dmul_rn(y, y)),
+                             bad ? CUDART_INF : 0.0);
   }
 }
 
@@ -721,7 +730,7 @@ __global__ void __launch_bounds__(MR_THREADS, CPL *NPOL <= 4 ? 2 : 1)
       for (int rd = 0; rd < n_rounds; ++rd) {
         // ---- stage one sample per lane
         int key = -1;
-        bool inf = false;
+        bool inf = false;  // a value or a tap of the sample is not finite
         if (raw.ok) {
           const Rec rc = raw.rc;
           const uint32_t tb = fdiv(rc.row, t.div_nchan);
@@ -731,7 +740,7 @@ __global__ void __launch_bounds__(MR_THREADS, CPL *NPOL <= 4 ? 2 : 1)
           const bool has = cfb >= 0 && cfb < a.n_cfb && cfc >= 0 && cfc < a.n_cfc;
           const int ou = min(max((int)rc.ou - 128 - q.first, 0), q.n_off - 1);
           const int ov = min(max((int)rc.ov - 128 - q.first, 0), q.n_off - 1);
-          if (!MULTI) tr[lane] = 0;
+          if (!MULTI) tr[lane] = q.zero_row;
 #pragma unroll
           for (int p = 0; p < NPOL; ++p) {
             double2 d;
@@ -740,18 +749,19 @@ __global__ void __launch_bounds__(MR_THREADS, CPL *NPOL <= 4 ? 2 : 1)
                                   __dmul_rn(raw.v[p].y, raw.w[p]));
             bool ok = has && lanes.ipm[p] >= 0 && !isnan(d.x) && !isnan(d.y) &&
                       (d.x != 0.0 || d.y != 0.0);
-            int row = 0;
+            int row = q.zero_row;
             if (ok) {
               const int64_t fidx = ((int64_t)cfb * a.n_cfc + cfc) * a.n_cfp + cfp[p];
               const int su = a.support[2 * fidx], sv = a.support[2 * fidx + 1];
               // a window larger than the plan's footprint (max_support) is skipped
               ok = su >= 1 && sv >= 1 && su <= S && sv <= S;
-              row = (int)((fidx * q.n_off + ou) * q.n_off + ov);
+              if (ok) row = (int)((fidx * q.n_off + ou) * q.n_off + ov);
             }
             wd[p * MR_ROUND + lane] = ok ? d : make_double2(0.0, 0.0);
             if (ok) {
-              sw[p] += __dmul_rn(raw.w[p], __ldg(q.norm + row));
-              inf |= isinf(d.x) || isinf(d.y);
+              const double2 nm = __ldg(q.norm + row);
+              sw[p] += __dmul_rn(raw.w[p], nm.x);
+              inf |= !(fabs(d.x) + fabs(d.y) + nm.y < CUDART_INF);
             }
             if (MULTI || ok) tr[(MULTI ? p : 0) * MR_ROUND + lane] = row;
           }
@@ -796,13 +806,15 @@ __global__ void __launch_bounds__(MR_THREADS, CPL *NPOL <= 4 ? 2 : 1)
             }
           }
         } else {
-          for (int j = 0; j < jn; ++j) {  // a round with an infinite value
+          for (int j = 0; j < jn; ++j) {
             if ((starts >> j) & 1u) {
               if (cur >= 0) lanes.flush(sre, sim, cur, m);
               cur = __shfl_sync(0xffffffffu, key, j);
             }
 #pragma unroll
-            for (int p = 0; p < NPOL; ++p)
+            for (int p = 0; p < NPOL; ++p) {
+              const double2 d = wd[p * MR_ROUND + j];
+              if (d.x == 0.0 && d.y == 0.0) continue;  // skipped: its row may be the zeros
 #pragma unroll
               for (int c = 0; c < CPL; ++c) {
                 const int row = tr[(MULTI ? p : 0) * MR_ROUND + j], i = lane + 32 * c;
@@ -811,8 +823,9 @@ __global__ void __launch_bounds__(MR_THREADS, CPL *NPOL <= 4 ? 2 : 1)
                 if (lanes.own[c] &&
                     mosaic_tap(a, row / per, S, i / S, i % S, q.first + row / q.n_off % q.n_off,
                                q.first + row % q.n_off, at))
-                  lanes.add(c, p, __ldg(a.cf + at), wd[p * MR_ROUND + j]);
+                  lanes.add(c, p, __ldg(a.cf + at), d);
               }
+            }
           }
         }
         __syncwarp();
@@ -857,7 +870,7 @@ __global__ void __launch_bounds__(MR_THREADS, CPL *NPOL <= 4 ? 2 : 1)
   }
 }
 
-static int64_t mosaic_tap_rows(int64_t n_cf, int os) { return n_cf * (os + 1) * (os + 1); }
+static int64_t mosaic_tap_rows(int64_t n_cf, int os) { return n_cf * (os + 1) * (os + 1) + 1; }
 
 static size_t mosaic_runs_smem(int S, int64_t n_img_pol, int npol_t) {
   const size_t stage = (size_t)MR_WARPS * MR_ROUND * npol_t * (sizeof(double2) + sizeof(int));
@@ -1161,7 +1174,7 @@ size_t av_mosaic_taps_size(int64_t n_cf, int max_support, int oversampling) {
   if (n_cf < 1 || max_support < 1 || oversampling < 1) return 0;
   const size_t rows = (size_t)mosaic_tap_rows(n_cf, oversampling);
   return Workspace::need(rows * max_support * max_support * sizeof(double2)) +
-         Workspace::need(rows * sizeof(double));
+         Workspace::need(rows * sizeof(double2));
 }
 
 int av_mosaic_runs_execute(AV_MOSAIC_PARAMS, void *workspace, size_t workspace_bytes, void *taps,
@@ -1214,12 +1227,13 @@ int av_mosaic_runs_execute(AV_MOSAIC_PARAMS, void *workspace, size_t workspace_b
   t.chunk = std::max<int64_t>(1024, (rows + parts - 1) / parts);
   Workspace tw(taps, taps_bytes);
   double2 *tab = tw.take<double2>((size_t)rows_t * max_support * max_support);
-  double *norm = tw.take<double>((size_t)rows_t);
+  double2 *norm = tw.take<double2>((size_t)rows_t);
   q.taps = tab;
   q.norm = norm;
   // floor((u - u_pos) os + 0.5) with |u - u_pos| <= 0.5
   q.first = -(os_u / 2);
   q.n_off = os_u + 1;
+  q.zero_row = (int)(rows_t - 1);
   cudaStream_t st = as_stream(stream);
   k_mosaic_taps<<<(unsigned)rows_t, 128, 0, st>>>(t.m, max_support, q.first, q.n_off, tab, norm);
   AV_LAUNCH_CHECK();
