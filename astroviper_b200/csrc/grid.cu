@@ -340,6 +340,18 @@ __device__ void build_tap_tables64(double *tab, double *rs, const double *cgk, i
   }
 }
 
+// Whether a tap of the tables just built is not finite (the whole block calls
+// this).  A skipped sample and an empty group slot are zero values, whose
+// products with such taps are NaN where the reference forms none; the FP64
+// sources then go sample by sample without the zeros, and the adjoint sample
+// by sample, as in its row lanes.
+__device__ __forceinline__ bool taps_not_finite(const double *rs) {
+  __syncthreads();
+  bool bad = false;
+  for (int o = threadIdx.x; o < 256; o += blockDim.x) bad |= !isfinite(rs[o]);
+  return __syncthreads_or(bad) != 0;
+}
+
 // One staged sample in registers (loads in flight until used).
 template <int NPOL>
 struct Pref {
@@ -516,6 +528,8 @@ struct RowLanes {
   }
 
   // Staged samples [j, j1) of the current round, all in the current cell.
+  // SKIP: leaves zero values out.
+  template <bool SKIP>
   __device__ __forceinline__ void run(int j, int j1, const double2 *wd, const int *wm,
                                       const double *tab) {
     for (; j < j1; ++j) {
@@ -538,6 +552,7 @@ struct RowLanes {
 #pragma unroll
       for (int pp = 0; pp < PPL; ++pp) {
         const double2 d = wd[(pg * PPL + pp) * C::SDS + j];
+        if (SKIP && d.x == 0.0 && d.y == 0.0) continue;
         const double tr = cu * d.x, ti = cu * d.y;
 #pragma unroll
         for (int k = 0; k < KC; ++k) {
@@ -622,6 +637,28 @@ struct MmaLanes {
       for (int p = 0; p < NPOL; ++p) {
         const double2 d = wd[p * C::SDS + s];
         mma_f64_m16n8k4(acc[p], cu * d.x, cu * d.y, cv);
+      }
+    }
+  }
+
+  // Samples [j, j1) one by one in the same accumulators.  SKIP: leaves zero
+  // values out.
+  template <bool SKIP>
+  __device__ __forceinline__ void run_exact(int j, int j1, const double2 *wd, const int *wm,
+                                            const double *tab) {
+    for (; j < j1; ++j) {
+      const int ro = wm[j];
+      const double cu = tab[(ro & 0xffff) + g];
+      const double *cv = tab + (ro >> 16) + 2 * t;
+#pragma unroll
+      for (int p = 0; p < NPOL; ++p) {
+        const double2 d = wd[p * C::SDS + j];
+        if (SKIP && d.x == 0.0 && d.y == 0.0) continue;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          acc[p][q] = fma(cu * d.x, cv[q], acc[p][q]);
+          acc[p][2 + q] = fma(cu * d.y, cv[q], acc[p][2 + q]);
+        }
       }
     }
   }
@@ -773,6 +810,7 @@ __global__ void __launch_bounds__(GCfg<S, NPOL>::THREADS, 1) k_grid_tiled(TiledG
     const int i = i0 + threadIdx.x;
     if (i < 2 * npg * C::PS) sre[i] = 0.0;
   }
+  const bool exact = SRC == SRC_F64 && taps_not_finite(rs);
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // image polarisation of each visibility polarisation (-1 drops it)
@@ -864,7 +902,8 @@ __global__ void __launch_bounds__(GCfg<S, NPOL>::THREADS, 1) k_grid_tiled(TiledG
           }
           const unsigned later = j < 31 ? (starts & (0xfffffffeu << j)) : 0u;
           const int j1 = later ? min(jn, __ffs(later) - 1) : jn;
-          lanes.run(j, j1, wd, wm, tab);
+          if (exact) lanes.template run<true>(j, j1, wd, wm, tab);
+          else lanes.template run<false>(j, j1, wd, wm, tab);
           j = j1;
         }
         __syncwarp();
@@ -1011,6 +1050,7 @@ __global__ void __launch_bounds__(MCfg<S, NPOL, SRC>::THREADS, 1) k_grid_mma(Til
     const int i = i0 + threadIdx.x;
     if (i < 2 * npg * C::PS) sre[i] = 0.0;
   }
+  const bool exact = SRC != SRC_F32 && taps_not_finite(rs);
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int pm[NPOL];
@@ -1138,7 +1178,7 @@ __global__ void __launch_bounds__(MCfg<S, NPOL, SRC>::THREADS, 1) k_grid_mma(Til
         // ---- compute the round's samples in runs of one cell
         const int jn = (int)min((uint32_t)GT_STAGE, w_hi - (w_lo + (uint32_t)rd * GT_STAGE));
         int j = 0;
-        if (starts <= 1u && jn == GT_STAGE) {  // one run over the whole round
+        if (!exact && starts <= 1u && jn == GT_STAGE) {  // one run over the whole round
           if (starts) {
             if (cur >= 0) lanes.template flush<DET>(sre, sim, cur, dscale);
             cur = __shfl_sync(0xffffffffu, my_key, 0);
@@ -1153,7 +1193,8 @@ __global__ void __launch_bounds__(MCfg<S, NPOL, SRC>::THREADS, 1) k_grid_mma(Til
           }
           const unsigned later = j < 31 ? (starts & (0xfffffffeu << j)) : 0u;
           const int j1 = later ? min(jn, __ffs(later) - 1) : jn;
-          lanes.run(j, j1, slot, wm, tab);
+          if (exact) lanes.template run_exact<SRC == SRC_F64>(j, j1, slot, wm, tab);
+          else lanes.run(j, j1, slot, wm, tab);
           j = j1;
         }
         __syncwarp();
