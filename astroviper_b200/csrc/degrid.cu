@@ -215,7 +215,11 @@ struct DSmem {
   static constexpr size_t total = tab_bytes + rs_bytes + sub_bytes;
 };
 
-template <int S, int RW>
+// FP32 taps of offset o - 128 and their FP64 sum rs[o] (RECIPROCAL: 1 / sum,
+// infinite for a zero sum).  The sum is the rounded taps' own, so a constant
+// grid degrids to itself: with the unrounded taps' sum the error of cubes of
+// 0.9M samples against FP64 is 4 % larger.
+template <int S, int RW, bool RECIPROCAL>
 __device__ void build_tap_tables_d(float *tab, double *rs, const double *cgk, int cgk_len,
                                    int os) {
   for (int o = threadIdx.x; o < 256; o += blockDim.x) {
@@ -228,11 +232,12 @@ __device__ void build_tap_tables_d(float *tab, double *rs, const double *cgk, in
         int k = os * (i - S / 2) + off;
         k = k < 0 ? -k : k;
         v = (k < cgk_len) ? cgk[k] : 0.0;
-        s += v;
       }
-      tab[o * RW + i] = (float)v;
+      const float t = (float)v;
+      tab[o * RW + i] = t;
+      s += (double)t;
     }
-    rs[o] = s;
+    rs[o] = RECIPROCAL ? 1.0 / s : s;
   }
 }
 
@@ -380,14 +385,16 @@ __device__ __forceinline__ uint32_t load_flags(const TiledDegridArgs &a, uint32_
   return v;
 }
 
-// STORE: writes one sample's values, already normalised; zeros for flagged,
-// unmapped and marked ones (k_degrid_exceptions then writes the marked
-// samples that the degridder keeps).
+// STORE: writes one sample's values, scaled in FP64 by inv = 1 / norm; zeros
+// for flagged, unmapped, zero-norm (inv infinite) and marked ones
+// (k_degrid_exceptions then writes the marked samples that the degridder
+// keeps).
 template <int NPG>
 __device__ __forceinline__ void store_values(const TiledDegridArgs &a, const int (&pmv)[8],
                                              uint32_t row, bool marked, uint32_t flags,
-                                             const float2 (&acc)[NPG]) {
+                                             double inv, const float2 (&acc)[NPG]) {
   const DegridArgs &d = a.d;
+  const bool keep = !marked && !isinf(inv);
   float2 v[4];
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
@@ -396,7 +403,9 @@ __device__ __forceinline__ void store_values(const TiledDegridArgs &a, const int
 #pragma unroll
     for (int gp = 1; gp < NPG; ++gp)
       if (apol == gp) x = acc[gp];
-    v[p] = apol >= 0 && !marked && ((flags >> (8 * p)) & 255u) == 0u ? x : make_float2(0.f, 0.f);
+    v[p] = apol >= 0 && keep && ((flags >> (8 * p)) & 255u) == 0u
+               ? make_float2((float)((double)x.x * inv), (float)((double)x.y * inv))
+               : make_float2(0.f, 0.f);
   }
   float2 *o = (float2 *)d.values + (int64_t)row * d.nvpol;
   if (d.nvpol == 1) {
@@ -451,12 +460,13 @@ __device__ __forceinline__ void stage_subgrid(const DegridArgs &d, float2 *sub, 
   }
 }
 
-// STORE (complex64 store mode without phase): tap tables divided by their
-// sums, so no sample needs its norm, an FP64 divide and FP64 products; flags
-// read at the start of a step, their latency behind the footprint's sums; one
-// store per sample: 2.06M flagged samples of 2 polarisations 130 -> 88 us,
-// 4.16M of one polarisation 103 -> 93 (82 and 89 with the chunks in turn),
-// with the error against FP64 6.4e-8 (6.8e-8 with a norm per sample).
+// STORE (complex64 store mode without phase): reciprocals of the taps' sums in
+// the table, so no sample needs an FP64 divide; flags read at the start of a
+// step, their latency behind the footprint's sums; one store per sample:
+// 2.06M flagged samples of 2 polarisations 130 -> 84 us, 4.16M of one
+// polarisation 103 -> 87, with the error against FP64 of a divide per sample.
+// (Taps divided by their sums and no scaling at all: 81 and 91 us, but a
+// norm that is rounded to FP32 with them.)
 template <int S, int NPG, bool STORE>
 __global__ void __launch_bounds__(DT_THREADS) k_degrid_tiled(TiledDegridArgs a) {
   using M = DSmem<S, NPG>;
@@ -471,8 +481,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_degrid_tiled(TiledDegridArgs a) 
   const uint32_t n_rec = *a.n_rec;
   const uint32_t n_all = a.accumulate ? n_rec : (uint32_t)a.n_rows;
   const int64_t n_chunks = ((int64_t)n_all + a.chunk - 1) / a.chunk;
-  if (STORE) build_norm_tap_tables<S, RW>(tab, d.cf, a.cgk_len, d.sampling);
-  else build_tap_tables_d<S, RW>(tab, rs, d.cf, a.cgk_len, d.sampling);
+  build_tap_tables_d<S, RW, STORE>(tab, rs, d.cf, a.cgk_len, d.sampling);
   int pmv[8];
 #pragma unroll
   for (int p = 0; p < 8; ++p) {
@@ -624,8 +633,8 @@ __global__ void __launch_bounds__(DT_THREADS) k_degrid_tiled(TiledDegridArgs a) 
         }
       }
       if (STORE) {
-        store_values<NPG>(a, pmv, ra.row, ma, fa, acca);
-        if (has_b) store_values<NPG>(a, pmv, rcb.row, mb, fb, accb);
+        store_values<NPG>(a, pmv, ra.row, ma, fa, rs[ra.ou] * rs[ra.ov], acca);
+        if (has_b) store_values<NPG>(a, pmv, rcb.row, mb, fb, rs[rcb.ou] * rs[rcb.ov], accb);
       } else {
         degrid_write<NPG>(a, d, rs, pmv, ra, ma, acca);
         if (has_b) degrid_write<NPG>(a, d, rs, pmv, rcb, mb, accb);
