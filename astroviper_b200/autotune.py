@@ -31,7 +31,7 @@ from ._lib import (AV_DEGRID_LANES_FP32, AV_DEGRID_LANES_TF32, AV_GRID_LANES_MMA
                    AV_GRID_LANES_ROWS, AV_TUNE_DEGRID_CHUNKS_PER_SM, AV_TUNE_DEGRID_LANES,
                    AV_TUNE_GRID_CHUNKS_PER_SM, AV_TUNE_GRID_LANES, check, lib)
 
-CANDIDATES = (4, 8, 16, 32, 64)  # record chunks per SM
+CANDIDATES = (4, 8, 16, 32, 64)  # of the chunks-per-SM knobs (include/av200.h)
 # kernel -> ((knob name, knob id, candidate values), ...), timed as a product
 SPACES = {
     "grid": (("lanes", AV_TUNE_GRID_LANES, (AV_GRID_LANES_MMA, AV_GRID_LANES_ROWS)),

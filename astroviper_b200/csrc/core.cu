@@ -104,7 +104,7 @@ __global__ void k_pswf_kernel4d(double *out, int os, int support, int n_os) {
 // ------------------------------------------------------------ tuning ---
 constexpr int kTuneKnobs = 5;
 static std::atomic<int64_t> g_tune[kTuneKnobs] = {
-    {8}, {16}, {AV_GRID_LANES_AUTO}, {AV_DEGRID_LANES_AUTO}, {2000000}};
+    {16}, {16}, {AV_GRID_LANES_AUTO}, {AV_DEGRID_LANES_AUTO}, {2000000}};
 
 int64_t tune_value(int knob) {
   return (knob >= 0 && knob < kTuneKnobs) ? g_tune[knob].load() : 0;

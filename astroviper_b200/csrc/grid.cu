@@ -1282,10 +1282,10 @@ static int dispatch_npol(const TiledGridArgs &a, int npol, int64_t nb, cudaStrea
 }
 
 // Chunks of records the persistent CTAs take one at a time: the same number
-// for each SM, up to AV_TUNE_GRID_CHUNKS_PER_SM (8), of at most 2048 records
-// below that, so that a chunk's tile flushes stay small against its samples
-// and the CTAs finish together.  With the long chunks taken first, 8 do
-// better than 16: 4.2M samples of one polarisation 144 -> 126 us, 128 planes
+// for each SM, up to half of AV_TUNE_GRID_CHUNKS_PER_SM (16, set when chunks
+// were taken in record order), of at most 2048 records below that, so that a
+// chunk's tile flushes stay small against its samples and the CTAs finish
+// together.  With the long chunks taken first, 8 do better than 16: 4.2M samples of one polarisation 144 -> 126 us, 128 planes
 // 1672 -> 1656, 33M samples 1588 -> 1586.  Up to one chunk of 2048 for each SM
 // the samples are spread over all SMs: 100,800 samples 37.6 us in 50 chunks,
 // 27.4 in 99 of 1024 or 132 of 768, 29.5 in 197 of 512 (two rounds).  Whole
@@ -1293,7 +1293,7 @@ static int dispatch_npol(const TiledGridArgs &a, int npol, int64_t nb, cudaStrea
 // 2048 127 us).
 static int64_t grid_chunking(int64_t rows, int64_t &nblocks) {
   const int sms = sm_count();
-  const int64_t per_sm = tune_value(AV_TUNE_GRID_CHUNKS_PER_SM);
+  const int64_t per_sm = std::max<int64_t>(1, tune_value(AV_TUNE_GRID_CHUNKS_PER_SM) / 2);
   const int64_t turns = std::min(per_sm, std::max<int64_t>(1, (rows + (int64_t)sms * 2048 - 1) /
                                                                   ((int64_t)sms * 2048)));
   int64_t chunk = (rows + sms * turns - 1) / (sms * turns);

@@ -61,10 +61,14 @@ unsigned long long av_launch_count(void);
 /* Launch tuning (no counterpart in the reference, which has no GPU path):
  * process-wide knobs read when a kernel is launched, set by the autotuner
  * (astroviper_b200.autotune) or by hand.
- *   AV_TUNE_GRID_CHUNKS_PER_SM   record chunks per SM handed out by the
- *                                persistent tiled gridder (default 8)
+ *   AV_TUNE_GRID_CHUNKS_PER_SM   bounds the record chunks per SM handed out
+ *                                by the persistent tiled gridder: at most
+ *                                half as many (at least one), fewer for few
+ *                                samples (default 16)
  *   AV_TUNE_DEGRID_CHUNKS_PER_SM record chunks per SM handed out by the
- *                                persistent tiled degridder (default 16)
+ *                                persistent tiled degridder (default 16); its
+ *                                FP32 kernel takes half as many (at least
+ *                                one)
  *   AV_TUNE_GRID_LANES           how the tiled gridder sums a run of samples:
  *                                AV_GRID_LANES_MMA (FP64 tensor-core tiles,
  *                                supports up to 8), AV_GRID_LANES_ROWS (a
