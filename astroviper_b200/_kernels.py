@@ -73,19 +73,29 @@ def on_device(x, dtype=None):
 _NP_OF = {torch.float64: np.float64, torch.int32: np.int32}
 
 
+def _packable(x):
+    """Whether upload packs x: an array of real numbers that torch takes too
+    (not one of strings, objects, dates, foreign bytes or negative strides)."""
+    return (isinstance(x, np.ndarray) and x.dtype.kind in "fiub" and x.dtype.itemsize <= 8
+            and x.dtype.isnative and min(x.strides, default=0) >= 0)
+
+
 def upload(*items):
     """Contiguous CUDA tensors of (array or tensor, dtype) pairs, dtype
     float64 or int32.  The host arrays among them (frequencies, channel and
     polarisation maps: a few hundred bytes each) go up together, in one
     asynchronous copy from page-locked memory; one copy each from pageable
-    memory made the host wait for every one of them."""
+    memory made the host wait for every one of them.  Everything else goes
+    through on_device, which refuses what it always has: copies of host
+    arrays in a graph capture too."""
     out = [None] * len(items)
     pack, size = [], 0
+    capturing = torch.cuda.is_current_stream_capturing()
     for i, (x, dt) in enumerate(items):
-        if isinstance(x, torch.Tensor):
+        if capturing or not _packable(x):
             out[i] = on_device(x, dt)
         else:
-            a = np.ascontiguousarray(np.asarray(x), dtype=_NP_OF[dt])
+            a = np.ascontiguousarray(x, dtype=_NP_OF[dt]).reshape(x.shape)
             pack.append((i, a, size))
             size += (a.nbytes + 15) & ~15
     if size == 0:
