@@ -806,6 +806,17 @@ def mosaic_tiled_ok(support, oversampling, n_img_pol):
             and int(np.min(np.asarray(support))) >= 1)
 
 
+def mosaic_runs_ok(n_cf, cu, cv, max_support, oversampling, npol):
+    """Whether mosaic_grid runs the kernel with the footprint in registers:
+    windows of up to 11 cells and 4 polarisations, unless gathering the taps
+    of every kernel offset would be more work than reading the functions a
+    few times (windows much wider than the support) or their rows, with one of
+    zeros, pass 31 bits."""
+    rows = n_cf * (oversampling + 1) ** 2
+    return (max_support <= 11 and npol <= 4 and rows < 0x7fffffff
+            and rows * max_support ** 2 <= 4 * n_cf * cu * cv + (1 << 20))
+
+
 def mosaic_grid(grid, sum_weight, do_psf, vis, weight, uvw, freq, chan_map, pol_map, cfb_map,
                 cfc_map, cfp_map, cf, support, n_uv, delta_lm, oversampling, aperture=False,
                 tiled=None):
@@ -846,12 +857,8 @@ def mosaic_grid(grid, sum_weight, do_psf, vis, weight, uvw, freq, chan_map, pol_
                                      float(delta_lm[0]), float(delta_lm[1]), max_sup, os_u, nt,
                                      nb, nchan, n_img_chan, wptr, wbytes, stream_ptr()),
           "av_mosaic_tiled_plan")
-    # the kernel with the footprint in registers, unless gathering the taps of
-    # every kernel offset would be more work than reading the functions a few
-    # times (windows much wider than the support), or has no room
     n_cf = n_cfb * n_cfc * n_cfp
-    taps = n_cf * (os_u + 1) ** 2 * max_sup ** 2
-    if max_sup <= 11 and npol <= 4 and taps <= 4 * n_cf * cu * cv + (1 << 20):
+    if mosaic_runs_ok(n_cf, cu, cv, max_sup, os_u, npol):
         tab = _scratch(lib().av_mosaic_taps_size(n_cf, max_sup, os_u))
         if tab is not None:
             check(lib().av_mosaic_runs_execute(*args, wptr, wbytes, tab[1], tab[2],

@@ -1,0 +1,12 @@
+"""Which mosaic calls take the kernel with the footprint in registers (no GPU)."""
+import pytest
+
+
+@pytest.mark.parametrize("args,want", [
+    ((6, 32, 32, 7, 4, 2), True), ((6, 48, 48, 11, 4, 4), True), ((6, 52, 52, 12, 4, 2), False),
+    ((6, 32, 32, 7, 4, 5), False), ((600, 8, 8, 3, 20, 1), False),
+    # one-cell windows at every offset: the kernel's 31-bit row numbers
+    (((2**31 - 2) // 4, 2, 2, 1, 1, 1), True), ((2**31 // 4, 2, 2, 1, 1, 1), False)])
+def test_route(args, want):
+    from astroviper_b200 import _kernels as K
+    assert K.mosaic_runs_ok(*args) is want
