@@ -487,7 +487,7 @@ def grid_to_image(grid_t, sum_weight=None, apply_corr=True, out_dtype=None):
     if sum_weight is not None:
         sw = on_device(sum_weight, torch.float64).reshape(-1)
         assert sw.numel() == npl
-    ws = lib().av_grid_to_image_workspace_size(npl, nx, ny)
+    ws = lib().av_real_fft_workspace_size(npl, nx, ny, 1)
     _buf, wptr, wbytes = workspace(ws)
     check(lib().av_grid_to_image(p(g), dcode(g), p(sw), p(img), dcode(img), npl, nx, ny,
                                  int(bool(apply_corr)), wptr, wbytes, stream_ptr()),
@@ -520,7 +520,7 @@ def _real_fft_shifted(t):
     nx, ny = int(t.shape[-2]), int(t.shape[-1])
     npl = int(t.numel() // (nx * ny))
     out = torch.empty(t.shape, dtype=torch.complex128, device=t.device)
-    _buf, wptr, wbytes = workspace(lib().av_grid_to_image_workspace_size(npl, nx, ny))
+    _buf, wptr, wbytes = workspace(lib().av_real_fft_workspace_size(npl, nx, ny, 0))
     check(lib().av_image_to_grid(p(t), AV_F64, p(out), AV_C128, npl, nx, ny, 0, wptr, wbytes,
                                  stream_ptr()), "av_image_to_grid")
     return out

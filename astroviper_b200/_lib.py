@@ -89,6 +89,7 @@ SIGNATURES = {
                              _vp, _sz, _vp]),
     "av_fft_workspace_size": (_sz, [_i64, _i64, _i64, _i]),
     "av_grid_to_image_workspace_size": (_sz, [_i64, _i64, _i64]),
+    "av_real_fft_workspace_size": (_sz, [_i64, _i64, _i64, _i]),
     "av_grid_to_image": (_i, [_vp, _i, _vp, _vp, _i, _i64, _i64, _i64, _i, _vp, _sz, _vp]),
     "av_image_to_grid": (_i, [_vp, _i, _vp, _i, _i64, _i64, _i64, _i, _vp, _sz, _vp]),
     "av_fft_shifted": (_i, [_vp, _vp, _i, _i64, _i64, _i64, _i, _vp, _sz, _vp]),

@@ -422,13 +422,16 @@ size_t av_fft_workspace_size(int64_t nplanes, int64_t nx, int64_t ny, int precis
          Workspace::need(fft_work_bytes(nplanes, nx, ny, dbl ? FFT_Z2Z : FFT_C2C));
 }
 
-size_t av_grid_to_image_workspace_size(int64_t nplanes, int64_t nx, int64_t ny) {
-  // av_image_to_grid takes the same workspace
-  size_t buf = 0, inv = 0, fwd = 0;
+size_t av_real_fft_workspace_size(int64_t nplanes, int64_t nx, int64_t ny, int inverse) {
+  size_t buf = 0, work = 0;
   if (nplanes <= 0 || nx <= 0 || ny <= 0) return 0;
-  real_fft_need(nplanes, nx, ny, FFT_Z2D, &buf, &inv);
-  real_fft_need(nplanes, nx, ny, FFT_D2Z, &buf, &fwd);
-  return Workspace::need(buf) + Workspace::need(std::max(inv, fwd));
+  real_fft_need(nplanes, nx, ny, inverse ? FFT_Z2D : FFT_D2Z, &buf, &work);
+  return Workspace::need(buf) + Workspace::need(work);
+}
+
+size_t av_grid_to_image_workspace_size(int64_t nplanes, int64_t nx, int64_t ny) {
+  return std::max(av_real_fft_workspace_size(nplanes, nx, ny, 1),
+                  av_real_fft_workspace_size(nplanes, nx, ny, 0));
 }
 
 // The transform is always FP64: the grid correction divides by a taper

@@ -399,8 +399,13 @@ size_t av_fft_workspace_size(int64_t nplanes, int64_t nx, int64_t ny, int precis
  * sum_weight[p] for nplanes planes of (nx, ny).  grid AV_C64 or AV_C128;
  * the transform is always FP64 (cuFFT Z2D of the grid's Hermitian part, whose
  * transform is the real part); image AV_F32 or AV_F64.
- * sum_weight may be NULL (no division). apply_corr = 0 skips corrTerm. */
+ * sum_weight may be NULL (no division). apply_corr = 0 skips corrTerm.
+ * av_grid_to_image_workspace_size serves av_grid_to_image and
+ * av_image_to_grid; av_real_fft_workspace_size serves one of them (inverse =
+ * 1: av_grid_to_image) and makes that one's cuFFT plan only, so the first call
+ * on a new size does not wait for the other's. */
 size_t av_grid_to_image_workspace_size(int64_t nplanes, int64_t nx, int64_t ny);
+size_t av_real_fft_workspace_size(int64_t nplanes, int64_t nx, int64_t ny, int inverse);
 int av_grid_to_image(const void *grid, int grid_dtype, const double *sum_weight,
                      void *image, int image_dtype, int64_t nplanes, int64_t nx, int64_t ny,
                      int apply_corr, void *workspace, size_t workspace_bytes, void *stream);
