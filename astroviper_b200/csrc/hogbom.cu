@@ -949,7 +949,16 @@ static int launch_hogbom_reg(HogArgs<float> a, int tpr, int grid, cudaStream_t s
 }
 
 // k_hogbom_reg's smallest variant that holds the bands in registers; false
-// when none does (more than 2048 columns, 56 pixels a thread or 160 CTAs).
+// when none does (more than 2048 columns, 56 pixels a thread or 160 CTAs) or
+// k_hogbom is the faster: on tall narrow images whose width lets it take four
+// pixels per thread with no thread idle (a power of two).  There a row is too
+// short for a bulk copy to pay, and the variants of more than 14 rows per
+// thread spill.  200 iterations against k_hogbom: 256 columns, 15-50 rows per
+// thread 1.00-1.06 (14: 0.65); 128 columns, 16-56 rows 1.13-1.35 (14: 0.76);
+// 64 columns, 15-56 rows 1.38-1.89 (14: 0.92); 512 columns, 15 and 16 rows
+// 1.05, 20-56 rows 0.98-0.91; up to 32 columns, bands of 80 rows 0.97-1.02,
+// of 90 1.00-1.08, of 300 1.9-2.8.  Other widths take k_hogbom_reg to the end
+// (100 columns 0.48-0.23, 300 0.70-0.45, 450 0.89-0.44, 600-1024 0.65-0.41).
 static bool hogbom_reg(const HogArgs<float> &a, int grid, cudaStream_t st, int &rc) {
   if (a.nx > 4 * HOG_RT || grid > HOG_MAX_CTAS) return false;
   const int nc = a.nx <= HOG_RT ? 1 : (a.nx <= 2 * HOG_RT ? 2 : 4);
@@ -957,6 +966,9 @@ static bool hogbom_reg(const HogArgs<float> &a, int grid, cudaStream_t st, int &
   const int rg = HOG_RT / tpr, band = (a.ny + grid - 1) / grid;
   const int rj = (band + rg - 1) / rg;
   if (rj * nc > 56) return false;
+  const bool four_wide = a.nx >= 4 && a.nx <= 512 && (a.nx & (a.nx - 1)) == 0;
+  if (four_wide && ((rj > 14 && (a.nx < 512 || rj < 20)) || (a.nx <= 32 && band > 80)))
+    return false;
   if (nc == 1) {
     if (rj <= 1) rc = launch_hogbom_reg<1, 1>(a, tpr, grid, st);
     else if (rj <= 2) rc = launch_hogbom_reg<1, 2>(a, tpr, grid, st);
