@@ -175,6 +175,51 @@ def rel(a, b):
 # ---------------------------------------------------------------------------
 # CPU side (oracle port on the host cores)
 # ---------------------------------------------------------------------------
+def plain_grid(vis, weight, uvw, freq, chan_map, npol, cgk, img, cell, support, planes,
+               do_psf=False):
+    """(grid, sum of weights) by av_grid_plain, the reference's per-sample
+    arithmetic in FP64: no plan, tiles or tensor cores, which the kernels that
+    it checks share with precision="fp64"."""
+    import torch
+
+    from astroviper_b200 import _kernels as K
+    from astroviper_b200._lib import AV_C128, AV_F64, check, lib
+    nt, nb, nchan = (int(s) for s in weight.shape[:3])
+    nx, ny = int(img[0]), int(img[1])
+    grid = torch.zeros((planes, npol, nx, ny), dtype=torch.complex128, device=weight.device)
+    sums = torch.zeros((planes, npol), dtype=torch.float64, device=weight.device)
+    w = weight.to(torch.float64).contiguous()
+    v = None if do_psf else vis.to(torch.complex128).contiguous()
+    u, f, cm, pm, cf = K.upload((uvw, torch.float64), (freq, torch.float64),
+                                (chan_map, torch.int32), (np.arange(npol), torch.int32),
+                                (cgk, torch.float64))
+    check(lib().av_grid_plain(K.p(grid), AV_C128, K.p(sums), int(do_psf), 0, K.p(v), AV_C128,
+                              K.p(w), AV_F64, K.p(u), K.p(f), K.p(cm), K.p(pm), K.p(cf), nx, ny,
+                              float(cell[0]), float(cell[1]), support, 100, nt, nb, nchan, npol,
+                              planes, npol, K.stream_ptr()), "av_grid_plain")
+    return grid, sums
+
+
+def plain_degrid(grid, uvw, freq, chan_map, npol, cgk, img, cell, support):
+    """Values by av_degrid_plain, one thread per value in FP64."""
+    import torch
+
+    from astroviper_b200 import _kernels as K
+    from astroviper_b200._lib import AV_C128, check, lib
+    nt, nb, nchan = int(uvw.shape[0]), int(uvw.shape[1]), len(freq)
+    g = grid.to(torch.complex128).contiguous()
+    planes, g_npol, nx, ny = (int(s) for s in g.shape)
+    out = torch.zeros((nt, nb, nchan, npol), dtype=torch.complex128, device=g.device)
+    u, f, cm, pm, cf = K.upload((uvw, torch.float64), (freq, torch.float64),
+                                (chan_map, torch.int32), (np.arange(npol) % g_npol, torch.int32),
+                                (cgk, torch.float64))
+    check(lib().av_degrid_plain(K.p(u), None, K.p(out), AV_C128, None, -float(cell[0]) * nx,
+                                -float(cell[1]) * ny, nx / 2, ny / 2, K.p(g), AV_C128, planes,
+                                g_npol, nx, ny, K.p(f), K.C_LIGHT, support, 100, K.p(cf), K.p(cm),
+                                K.p(pm), nt, nb, nchan, npol, K.stream_ptr()), "av_degrid_plain")
+    return out
+
+
 def bench_config(world, n_time=None):
     """The workload description, the same in both arms."""
     n_vis = (n_time or N_TIME) * 2016 * 64
@@ -440,8 +485,8 @@ def main():
     pa = torch.cuda.Event(enable_timing=True)
     pb = torch.cuda.Event(enable_timing=True)
     pa.record()
-    g64, s64 = K.grid(vis_s, iw_s, uvw_s, W["freq"], np.zeros(nchan, int), np.arange(npol),
-                      G.cgk, img, cell, 7, 100, 1, npol, precision="fp64")
+    g64, s64 = plain_grid(vis_s, iw_s, uvw_s, W["freq"], np.zeros(nchan, int), npol, G.cgk, img,
+                          cell, 7, 1)
     pb.record()
     torch.cuda.synchronize()
     t_plain = pa.elapsed_time(pb)
@@ -455,17 +500,16 @@ def main():
     # PSF: the weights gridded (do_psf) and imaged, FP32-input tiled path
     # against the FP64 plain gridder
     p32, ps32 = Gs.grid(None, iw[:ts], do_psf=True)
-    p64, ps64 = K.grid(None, iw_s, uvw_s, W["freq"], np.zeros(nchan, int), np.arange(npol),
-                       G.cgk, img, cell, 7, 100, 1, npol, do_psf=True, precision="fp64")
+    p64, ps64 = plain_grid(None, iw_s, uvw_s, W["freq"], np.zeros(nchan, int), npol, G.cgk, img,
+                           cell, 7, 1, do_psf=True)
     pi32, pi64 = Gs.image(p32, ps32), Gs.image(p64, ps64)
     err_psf = rel(pi32, pi64)
     mx_psf = max_elem_err(pi32, pi64)
     del p32, p64, pi32, pi64
     v32 = Gs.degrid(g64)
     nx, ny = int(img[0]), int(img[1])
-    v64 = K.degrid(g64, uvw_s, W["freq"], (-cell[0] * nx, -cell[1] * ny), (nx / 2, ny / 2),
-                   (np.arange(nchan) / nchan * 1).astype(int), np.arange(npol) % npol, G.cgk, 7,
-                   100, nvchan=nchan, nvpol=npol, precision="fp64")
+    v64 = plain_degrid(g64, uvw_s, W["freq"], (np.arange(nchan) / nchan * 1).astype(int), npol,
+                       G.cgk, img, cell, 7)
     err_vis = rel(v32, v64)
     mx_vis = max_elem_err(v32, v64)
     del g64, v64, v32, vis_s
@@ -653,9 +697,8 @@ def bench_batched(args, dev):
         t64 = {}
 
         def fp64():
-            t64["g"], _ = K.grid(v64, w64, W["uvw"], W["freq"], np.arange(nchan), np.arange(npol),
-                                 cgk, W["image_size"], W["pixelincr"], support, 100, nchan, npol,
-                                 precision="fp64")
+            t64["g"], _ = plain_grid(v64, w64, W["uvw"], W["freq"], np.arange(nchan), npol, cgk,
+                                     W["image_size"], W["pixelincr"], support, nchan)
         r["fp64_plain_ms"] = timed(fp64, 1)
         r["rel_err_vs_fp64"] = rel(gb, t64["g"])
         r["speedup_vs_per_grid"] = r["per_grid_ms"] / r["graph_ms"]
