@@ -11,6 +11,7 @@
 // both halves of its spectrum.  Complex data go through Z2Z / C2C
 // (av_fft_shifted).
 #include <cufft.h>
+#include <math_constants.h>
 
 #include <algorithm>
 #include <deque>
@@ -155,12 +156,12 @@ __device__ __forceinline__ double corr_factor(int64_t i, int64_t n) {
   return pswf_grdsf(fabs(2.0 * ((double)(i - n / 2) / (double)n)));
 }
 
-// v / d for d near 1 / r (a few ulp), Markstein's correction ("Computation of
-// elementary functions on the IBM RISC System/6000 processor", 1990): one
-// Newton step makes r the rounded reciprocal, and the exact remainder of
-// v r corrects the quotient's last bit.  7 FP64 operations per pixel in place
-// of a divide's call; zeros, infinities, NaN and results whose remainder
-// could leave the normal range take the divide.
+// v / d for 1e-20 < |d| < 1e300 and r near 1 / d (a few ulp), by Markstein's
+// correction ("Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990): one Newton step makes r the rounded reciprocal, and the
+// exact remainder of v r corrects the quotient's last bit.  7 FP64 operations
+// per pixel in place of a divide's call; zeros, infinities, NaN and results
+// whose remainder could leave the normal range take the divide.
 __device__ __forceinline__ double quotient(double v, double d, double r) {
   r = fma(r, fma(-d, r, 1.0), r);
   double q = v * r;
@@ -169,7 +170,15 @@ __device__ __forceinline__ double quotient(double v, double d, double r) {
   return fma(fma(-q, d, v), r, q);
 }
 
-// v / d for r = 1 / d rounded: as above without the Newton step.
+// 1 / d rounded where quotient_by corrects its products; NaN, which sends
+// every quotient to the divide, for a d so small that a remainder could fall
+// below the normal range, or so large that 1 / d does.
+__device__ __forceinline__ double reciprocal_for_quotient(double d) {
+  const double m = fabs(d);
+  return m > 1e-20 && m < 1e300 ? 1.0 / d : CUDART_NAN;
+}
+
+// v / d for r = reciprocal_for_quotient(d): as above without the Newton step.
 __device__ __forceinline__ double quotient_by(double v, double d, double r) {
   const double q = v * r;
   const double m = fabs(q);
@@ -207,7 +216,7 @@ __device__ __forceinline__ void for_pixels(int64_t nplanes, int64_t nx, int64_t 
     if (j >= ny) continue;
     const int rows = (int)std::min<int64_t>(IMG_ROWS, nx - i0);
     for (int64_t p = blockIdx.z; p < nplanes; p += gridDim.z) {
-      const double sw = f.sumw ? f.sumw[p] : 1.0, rsw = 1.0 / sw;
+      const double sw = f.sumw ? f.sumw[p] : 1.0, rsw = reciprocal_for_quotient(sw);
       const auto *in = f.in + p * f.plane_in() + f.col_in(j);
       auto *out = f.out + p * f.plane_out() + f.col_out(j);
       for (int r = 0; r < rows; r += IMG_UNROLL) {
