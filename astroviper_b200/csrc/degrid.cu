@@ -197,7 +197,8 @@ struct TiledDegridArgs {
   uint32_t *sched;          // device: [0] next chunk, [1] CTAs done (0 between launches)
   int accumulate;           // 1: values +=, 0: values = (skipped samples get 0)
   // complex64 store mode, 4 visibility polarisations, no flags, no phase,
-  // values 32-byte aligned: a sample's 4 values go out as two 16-byte stores
+  // values 32-byte aligned: what the tensor-core kernels take (a sample's 4
+  // values go out as two 16-byte stores)
   int fast_out;
   // complex64 store mode, up to 4 visibility polarisations, no phase: the
   // STORE variant of k_degrid_tiled
@@ -303,35 +304,8 @@ __device__ __forceinline__ void degrid_write(const TiledDegridArgs &a, const Deg
     // a shared plan's sample whose degridder convention differs: zeros in
     // store mode (k_degrid_exceptions then writes the ones the degridder
     // keeps), nothing when accumulating
-    if (!a.accumulate) {
-      if (a.fast_out) {
-        float4 *o = (float4 *)((float2 *)d.values + row_i * 4);
-        o[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-        o[1] = make_float4(0.f, 0.f, 0.f, 0.f);
-      } else {
-        for (int p = 0; p < d.nvpol; ++p) put_value(d, 0, row_i * d.nvpol + p, 0.0, 0.0);
-      }
-    }
-    return;
-  }
-  if (a.fast_out) {
-    // 1 / norm in FP64, the scaling in FP32 (one more rounding, ~6e-8)
-    const float inv = norm != 0.0 ? (float)(1.0 / norm) : 0.f;
-    float2 v[4];
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      const int apol = pmv[p];
-      float2 x = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int gp = 0; gp < NPG; ++gp)
-        if (apol == gp) x = acc[gp];
-      // zero-norm samples and unmapped polarisations get 0, as in store mode
-      v[p] = (apol >= 0 && norm != 0.0) ? make_float2(__fmul_rn(x.x, inv), __fmul_rn(x.y, inv))
-                                        : make_float2(0.f, 0.f);
-    }
-    float4 *o = (float4 *)((float2 *)d.values + row_i * 4);
-    o[0] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
-    o[1] = make_float4(v[2].x, v[2].y, v[3].x, v[3].y);
+    if (!a.accumulate)
+      for (int p = 0; p < d.nvpol; ++p) put_value(d, 0, row_i * d.nvpol + p, 0.0, 0.0);
     return;
   }
   if (norm == 0.0) {  // the reference leaves such samples untouched
