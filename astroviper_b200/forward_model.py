@@ -87,8 +87,9 @@ class ForwardModel:
                                                                      torch.float64)
         grid = torch.empty(self.image_shape, dtype=torch.complex128, device=self.dev)
         npl = self.n_img_chan * self.n_img_pol
-        _buf, wptr, wbytes = K.workspace(lib().av_real_fft_workspace_size(npl, self.nx, self.ny,
-                                                                          0))
+        # both directions' plans are made here: the adjoint follows
+        _buf, wptr, wbytes = K.workspace(lib().av_grid_to_image_workspace_size(npl, self.nx,
+                                                                               self.ny))
         check(lib().av_image_to_grid(K.p(img), K.dcode(img), K.p(grid), AV_C128, npl, self.nx,
                                      self.ny, 1, wptr, wbytes, K.stream_ptr()),
               "av_image_to_grid")
