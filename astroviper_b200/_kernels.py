@@ -166,8 +166,8 @@ def degrid_tiled_ok(precision, support, sampling, g_npol, c):
 
 
 def _plan_us(rows, planes, nu, nv, support):
-    """Microseconds a binning plan costs (ten launches, 8 ps a cell key for its
-    scan, 50 ps a sample)."""
+    """Microseconds charged for binning a call: 40 for its six launches, 8 ps
+    a cell key for the scan, 50 ps a sample for the plan's two walks."""
     tiles = planes * (-(-(nu - support + 1) // 32)) * (-(-(nv - support + 1) // 32))
     return 40.0 + 8e-6 * 1024 * tiles + 5e-5 * rows
 
@@ -176,8 +176,14 @@ def _binning_pays(plain_ps, rows, npol, planes, nu, nv, support):
     """Whether binning the samples first beats the plain FP64 kernel, which
     takes plain_ps picoseconds a tap and correlation (33 for the gridder, 2.5
     for the degridder, 806k samples x 2 pol, support 7: 2620 and 199 us, binned
-    109 and 128 us with the plan).  The binned kernels' own time hides behind
-    the plan's.  The plan also has to fit its key and row ranges."""
+    96 and 127 us with the plan).  The binned kernels' own time is not charged;
+    a small call's host work is.  Both sides measured over 627 calls (1200 to
+    1.6M samples, 256^2 to 4096^2, supports 3-9, 1-4 polarisations): the side
+    taken is the slower one by more than 3 % in 37 of them.  Six are binned
+    (degridding 0.8M-1.6M samples 4-8 %, one small gridding call 16 %); the
+    others stay plain, most of them support 3, where the plain gridder's
+    atomics meet in few cells and cost more per tap (up to 4.6 times).  The
+    plan also has to fit its key and row ranges."""
     if (not 3 <= support <= 9 or nu < support or nv < support or max(nu, nv) >= 131072
             or rows >= 1 << 31):
         return False
@@ -203,8 +209,9 @@ def grid(vis, weight, uvw, freq, chan_map, pol_map, cgk, n_uv, delta_lm, support
 
     precision "fp32": the tiled kernel (reads complex64 visibilities and
     float32 weights, accumulates in FP64; complex128 grid unless a complex64
-    grid is passed); "fp64": the plain FP64 kernel (FP64 inputs, every option
-    of the reference, complex128 grid)."""
+    grid is passed); "fp64": FP64 inputs and arithmetic, every option of the
+    reference, complex128 grid, by the plain FP64 kernel or, for the tiled
+    kernel's shapes where _binning_pays, over binned samples."""
     dev = device()
     nu, nv = int(n_uv[0]), int(n_uv[1])
     nt, nb = int(uvw.shape[0]), int(uvw.shape[1])

@@ -1254,10 +1254,15 @@ static int launch_grid_mma(const TiledGridArgs &a, int64_t nblocks, cudaStream_t
 // 5-8: with smaller footprints most of the 8 x 8 tile is padding and the row
 // lanes are faster); k_grid_tiled otherwise (support 9).  The degridder's
 // adjoint follows the same rule: 4.16M samples of one polarisation, support 7,
-// take 126 us (145 in record order, the row lanes 210).  Double-precision inputs take
-// k_grid_mma for every support it covers, whatever the knob says: 806k
-// samples of 2 polarisations take 65 us, and 31 us of plan, against 2620 us of
-// k_grid_plain, whose 98 global FP64 atomics per correlation bound it.
+// take 122 us (145 in record order, the row lanes 210).
+// Double-precision inputs take k_grid_mma for every support it covers, whatever
+// the knob says: 806k samples of 2 polarisations, support 7, take 65 us, and
+// 31 us of plan, against 2620 us of k_grid_plain, whose 98 global FP64 atomics
+// per correlation bound it.  The row lanes there take, of k_grid_mma's time, at
+// 806k samples 1.05-1.3 (1 and 2 polarisations, supports 3-8; 4 polarisations:
+// 0.9 at support 3, 1.0 at 4 and 5, 1.07-1.3 above), at 50k-108k samples
+// 0.85-1.05, and 0.65-0.8 at support 3 with 4 polarisations: little of a call
+// that the plan and the launches make up for the most part.
 template <int S, int NPOL>
 static int launch_grid_tiled(const TiledGridArgs &a, int64_t nblocks, cudaStream_t st) {
   const bool f64 = a.wt64 != nullptr || a.vis64 != nullptr;

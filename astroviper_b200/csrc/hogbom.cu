@@ -505,6 +505,9 @@ __global__ void __launch_bounds__(HOG_THREADS, 1) k_hogbom(HogArgs<T> a) {
 //   - A thread owns RJ rows x NC columns of its CTA's band in registers, and a
 //     pixel costs a load, a multiply, a subtraction and a maximum.  The
 //     maximum's place is looked for afterwards, by the warps that hold it only.
+//     Up to 14 pixels a thread nothing spills; at 28 up to 56 bytes do, and at
+//     56, which 2048^2 takes, 388 bytes of spill loads (bulk copies; 604
+//     without) of the mask and addresses come from L1 in an iteration.
 //   - The PSF rows an iteration needs come to shared memory by bulk copies
 //     (one per row, an mbarrier per four steps), 115 KB in flight per SM;
 //     4-byte loads through L1 brought 11 bytes a clock (loads cannot be
@@ -515,9 +518,10 @@ __global__ void __launch_bounds__(HOG_THREADS, 1) k_hogbom(HogArgs<T> a) {
 //     an atomic maximum, an arrival count, its release and a read of the
 //     winner, and no line that all SMs poll.  Two sets of inboxes are used in
 //     turn: a CTA can be at most one exchange ahead of the slowest.
-//   - A wait gives up timeout_ns after its 256th failed poll (at the first with
-//     a bound of 0), sets the error flag and leaves; the others then run into
-//     their own bound.
+//   - An exchange gives up timeout_ns after its 257th failed poll, looked at in
+//     every 256th (at the first with a bound of 0), sets the error flag and
+//     leaves; the others then run into their own bound.  A bulk copy has
+//     HOG_COPY_NS, whatever timeout_ns is.
 // An iteration on 2048^2 takes 6.3 us (k_hogbom 10.2), of which the band pass
 // 2.4-3.2 (the PSF from L2 alone: 1.3), the exchange 1.8 and the skew between
 // the CTAs' windows the rest; on 512^2 3.4 us, 256^2 3.1 us, mostly exchange.

@@ -506,12 +506,16 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mosaic_tiled(MosaicTiledArgs 
 //   - lane l owns window cells l, l + 32, ... and keeps their sums for all
 //     polarisations while the samples stay in one cell: one tap load and 4
 //     NPOL DFMA per sample and owned cell, shared atomics only when the cell
-//     changes; four samples' taps are in flight whatever the runs.
+//     changes; two samples' taps are in flight whatever the runs (one where a
+//     sample has more than 4 loads per lane).
 // Cells past the window hold zero taps and skipped values are zeros, so
 // products that the reference does not form are zeros too, unless the other
 // factor is not finite: a round with an infinite value or a row that holds a
 // tap that is not finite (both rare) goes tap by tap and value by value.
-// 1.03M samples x 2 polarisations, supports 5-7: 1315 us before, 207 us now (and 45 us of plan).
+// 1.03M samples x 2 polarisations, supports 5-7: k_mosaic_tiled 1315 us, this
+// 178 us (and 45 us of plan): 87M warp instructions, 84 a sample, issued in 47 %
+// of the cycles at 16 warps per SM (114 registers), which wait for fixed
+// latencies, taps and slots.
 constexpr int MR_MAX_S = 11;
 constexpr int MR_THREADS = 256;
 constexpr int MR_WARPS = MR_THREADS / 32;
@@ -651,8 +655,9 @@ __global__ void __launch_bounds__(MR_THREADS, CPL *NPOL <= 4 ? 2 : 1)
   const MosaicTiledArgs &t = q.t;
   const MosaicArgs &a = t.m;
   constexpr int NF = MULTI ? NPOL : 1;  // tap rows per sample
-  // samples whose taps are loaded together, up to 8 loads in flight per lane (2
-  // at a time take 225 us of the 1.03M samples, 4 256 us for their registers)
+  // samples whose taps are loaded together: two where a sample has up to 4
+  // loads per lane (225 us of the 1.03M samples with their chunks in record
+  // order; four at a time 256 us, for their registers), else one (up to 16)
   constexpr int AHEAD = NF * CPL <= 4 ? 2 : 1;
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -76,7 +76,8 @@ unsigned long long av_launch_count(void);
  *                                AV_GRID_LANES_AUTO (default: tensor-core
  *                                tiles for supports 5-8, where they are the
  *                                faster, rows otherwise); support 9 always
- *                                uses rows
+ *                                uses rows, and av_grid_double always
+ *                                tensor-core tiles for supports up to 8
  *   AV_TUNE_DEGRID_LANES         how the tiled degridder's fast store path
  *                                (complex64 values, 4 polarisations, no flags
  *                                or phase) runs: AV_DEGRID_LANES_TF32 (TF32
@@ -90,15 +91,21 @@ unsigned long long av_launch_count(void);
  *                                for 9)
  *   AV_TUNE_HOGBOM_BARRIER_TIMEOUT_US  how long (microseconds of wall time,
  *                                default 2000000) a CTA of av_hogbom_run
- *                                waits at the per-iteration grid barrier
- *                                before it gives up; on giving up the launch
- *                                ends, av_hogbom_state_read returns
- *                                AV_ERR_TIMEOUT ("grid barrier timed out")
- *                                and the run must be started again
- *                                (init_state = 1).  0 makes every CTA but
- *                                the last to arrive give up at its first
- *                                barrier, which is how the timeout path is
- *                                tested.  Range [0, 600000000].
+ *                                waits for the others in an iteration before
+ *                                it gives up: at the grid barrier of the
+ *                                shared-memory loop, or in the exchange of
+ *                                winners of the register-resident FP32 loop,
+ *                                which starts its clock at the 257th failed
+ *                                poll.  On giving up the launch ends,
+ *                                av_hogbom_state_read returns AV_ERR_TIMEOUT
+ *                                ("grid barrier timed out") and the run must
+ *                                be started again (init_state = 1).  With 0 a
+ *                                CTA gives up at its first failed look (at
+ *                                the barrier, every CTA but the last to
+ *                                arrive), which is how the timeout path is
+ *                                tested.  The register-resident loop's copies
+ *                                of PSF rows have a fixed bound of 2 s.
+ *                                Range [0, 600000000].
  * av_tune_set returns AV_ERR_ARG for an unknown knob or a value outside
  * [1, 1024] ([1, 3] for AV_TUNE_GRID_LANES, [1, 4] for AV_TUNE_DEGRID_LANES,
  * [0, 600000000] for the barrier timeout); av_tune_get returns -1 for an
