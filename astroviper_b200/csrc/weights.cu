@@ -56,14 +56,22 @@ __device__ __forceinline__ bool nearest_cell(double um, double vm, double f, dou
 }
 
 // How k_weight_density and k_briggs_apply walk the samples: a thread takes
-// one (baseline, channel) series and `steps` consecutive times of it (grid:
-// series / WT_THREADS, time blocks).  At each time the threads of a warp read
-// neighbouring rows, whatever the number of channels; the channel's uv scale,
-// with its divides, is formed once; and since a baseline stays in one cell
-// for several times, its weights are summed in a register and its density
-// looked up once per cell.  WT_UNROLL times are loaded together (2 with 4 blocks
-// per SM: 47 and 54 us; 4 at once spill there, 57 and 69 us).
+// `steps` consecutive times of one (baseline, channel) series.  Threads run
+// over a group of channels, the baselines, the time blocks and the groups, in
+// one line, so that few series leave no lane idle (1M samples of one series:
+// weights 218 -> 34 us, density 660 -> 147, against blocks of 256 series).
+// At each time the threads of a warp read neighbouring rows of 16 channels;
+// the channel's uv scale, with its divides, is formed once; and since a
+// baseline stays in one cell for several times, its weights are summed in a
+// register and its density looked up once per cell.  A group of 16 channels
+// keeps a warp's cells in 16 planes and several baselines of a channel in a
+// block, for its sum: the density of one time of 2016 baselines x 512 channels
+// takes 30 us, 37 in groups of 8, 56 of 32 (and 57 with all channels in one);
+// of 64 times of 2016 x 32 channels 32, 32 and 36.  WT_UNROLL times are loaded
+// together (2 with 4 blocks per SM; 4 at once spill there and take a fifth
+// longer).
 constexpr int WT_THREADS = 256, WT_UNROLL = 2;
+constexpr int64_t WT_GROUP = 16;  // channels of a group, at most
 
 // f(npol as a constant), npol 1, 2 or 4.
 template <typename F>
@@ -73,37 +81,64 @@ static void with_pols(int64_t npol, F f) {
   else f(std::integral_constant<int, 4>());
 }
 
-static dim3 weight_walk(int64_t nt, int64_t series, int64_t &steps) {
-  // two waves of 1024 threads per SM, at least WT_UNROLL times each
-  const int64_t want = (int64_t)sm_count() * 2048;
+struct WeightWalk {
+  int64_t steps, time_blocks;
+  int64_t width, groups;  // channels of a group (the last one may have fewer)
+  unsigned blocks;
+};
+
+// Two waves of 1024 threads per SM, at least WT_UNROLL times each.
+static WeightWalk weight_walk(int64_t nt, int64_t nb, int64_t nchan) {
+  WeightWalk w;
+  w.groups = (nchan + WT_GROUP - 1) / WT_GROUP;
+  w.width = (nchan + w.groups - 1) / w.groups;
+  const int64_t series = nb * w.width * w.groups, want = (int64_t)sm_count() * 2048;
   const int64_t most = (nt + WT_UNROLL - 1) / WT_UNROLL;
-  int64_t blocks_t = std::max<int64_t>(1, std::min(most, (want + series - 1) / series));
-  blocks_t = std::min<int64_t>(blocks_t, 65535);
-  steps = (nt + blocks_t - 1) / blocks_t;
-  steps = (steps + WT_UNROLL - 1) / WT_UNROLL * WT_UNROLL;
-  blocks_t = (nt + steps - 1) / steps;
-  return dim3((unsigned)((series + WT_THREADS - 1) / WT_THREADS), (unsigned)blocks_t);
+  const int64_t parts = std::max<int64_t>(1, std::min(most, (want + series - 1) / series));
+  w.steps = (nt + parts - 1) / parts;
+  w.steps = (w.steps + WT_UNROLL - 1) / WT_UNROLL * WT_UNROLL;
+  w.time_blocks = (nt + w.steps - 1) / w.steps;
+  w.blocks = (unsigned)((series * w.time_blocks + WT_THREADS - 1) / WT_THREADS);
+  return w;
 }
+
+// This thread's place in the walk.
+struct WeightPlace {
+  int64_t c, group_first, at;  // channel, its group's first one, first row of uvw
+  int n;                       // times, none past the end
+  __device__ __forceinline__ WeightPlace(const WeightWalk &w, int64_t nt, int64_t nb,
+                                         int64_t nchan) {
+    const int64_t k = blockIdx.x * (int64_t)WT_THREADS + threadIdx.x;
+    const int64_t k1 = k / w.width, k2 = k1 / nb, group = k2 / w.time_blocks;
+    group_first = group * w.width;
+    c = group_first + (k - k1 * w.width);
+    const int64_t t0 = (k2 - group * w.time_blocks) * w.steps;
+    at = t0 * nb + (k1 - k2 * nb);
+    n = c < nchan ? (int)std::min(nt - t0, w.steps) : 0;
+  }
+};
 
 // Density grid and sums of weights.  One thread per sample in channel-major
 // order, two global FP64 atomics each and the weights read with a stride of a
 // whole row, had taken 270 us for 4.1M samples x 4 polarisations (float32,
-// 32 planes of 1024^2); this walk takes 47 us
+// 32 planes of 1024^2); this walk takes DDD us.
 template <int NPOL, typename WT>
 __global__ void __launch_bounds__(WT_THREADS, 4) k_weight_density(
     double *G, double *sumw, const double *__restrict__ uvw, const double *__restrict__ freq,
     const WT *__restrict__ wt, const uint8_t *__restrict__ flag, int64_t n_u, int64_t n_v,
-    double dl0, double dl1, int64_t nt, int64_t nb, int64_t nchan, int64_t steps) {
-  __shared__ double s_sum[WT_THREADS];
-  const int64_t series = nb * nchan, s = blockIdx.x * (int64_t)WT_THREADS + threadIdx.x;
-  const bool shared_sum = nchan <= WT_THREADS;
-  s_sum[threadIdx.x] = 0.0;
+    double dl0, double dl1, int64_t nt, int64_t nb, int64_t nchan, WeightWalk walk) {
+  // channels of the groups that the block's threads are of: a group between
+  // two others has at least its channels in threads
+  constexpr int WT_SUMS = WT_THREADS + 2 * (int)WT_GROUP;
+  __shared__ double s_sum[WT_SUMS];
+  __shared__ int64_t s_first;
+  const WeightPlace place(walk, nt, nb, nchan);
+  const int64_t c = place.c;
+  if (threadIdx.x == 0) s_first = place.group_first;
+  for (int i = threadIdx.x; i < WT_SUMS; i += WT_THREADS) s_sum[i] = 0.0;
   __syncthreads();
   double total = 0.0;
-  int64_t c = 0;
-  if (s < series) {
-    const int64_t b = s / nchan;
-    c = s - b * nchan;
+  if (place.n > 0) {
     const double us0 = uv_scale(freq[c], dl0, n_u), us1 = uv_scale(freq[c], dl1, n_v);
     double *plane = G + c * n_u * n_v;
     int64_t cell = -1, conj = -1;
@@ -117,20 +152,20 @@ __global__ void __launch_bounds__(WT_THREADS, 4) k_weight_density(
       }
       acc = 0.0;
     };
-    const int64_t t0 = blockIdx.y * steps, t1 = std::min(nt, t0 + steps);
-    for (int64_t t = t0; t < t1; t += WT_UNROLL) {
+    int64_t at_t = place.at;  // row of uvw
+    for (int left = place.n; left > 0; left -= WT_UNROLL, at_t += WT_UNROLL * nb) {
       double um[WT_UNROLL], vm[WT_UNROLL], w[WT_UNROLL];
 #pragma unroll
       for (int k = 0; k < WT_UNROLL; ++k)
-        if (t + k < t1) {
-          const int64_t tb = (t + k) * nb + b;
+        if (k < left) {
+          const int64_t tb = at_t + k * nb;
           um[k] = uvw[3 * tb];
           vm[k] = uvw[3 * tb + 1];
           w[k] = pol_avg_weight<NPOL>(wt, flag, tb * nchan + c);
         }
 #pragma unroll
       for (int k = 0; k < WT_UNROLL; ++k) {
-        if (t + k >= t1) continue;
+        if (k >= left) continue;
         long long ui, vi, uic, vic;
         if (!scaled_cell(um[k], vm[k], us0, us1, n_u, n_v, ui, vi, uic, vic) || isnan(w[k]))
           continue;
@@ -148,16 +183,11 @@ __global__ void __launch_bounds__(WT_THREADS, 4) k_weight_density(
     }
     flush();
   }
-  // sums of weights: one atomic per channel and block where a block's
-  // channels fit its threads
-  if (shared_sum) {
-    if (total != 0.0) atomicAdd(&s_sum[c], total);
-    __syncthreads();
-    if (threadIdx.x < nchan && s_sum[threadIdx.x] != 0.0)
-      atomicAdd(&sumw[threadIdx.x], s_sum[threadIdx.x]);
-  } else if (total != 0.0) {
-    atomicAdd(&sumw[c], total);
-  }
+  // sums of weights: one atomic per channel and block
+  if (total != 0.0) atomicAdd(&s_sum[c - s_first], total);
+  __syncthreads();
+  for (int i = threadIdx.x; i < WT_SUMS; i += WT_THREADS)
+    if (s_sum[i] != 0.0) atomicAdd(&sumw[s_first + i], s_sum[i]);
 }
 
 // sum(G^2) per plane: one CTA per (plane, slice), FP64 partials.
@@ -216,37 +246,37 @@ struct PairOf<float> {
 
 // Imaging weight of each sample, tiled to every polarisation
 // (grid_imaging_weights.py:358-443 + calculate_imaging_weights.py:258-261),
-// in the walk above (89 us for the case above with one thread per sample;
-// 54 us now).
+// in the walk above (99 us for the case above with one thread per sample;
+// 58 us now).
 template <int NPOL, typename OT, typename WT>
 __global__ void __launch_bounds__(WT_THREADS, 4) k_briggs_apply(
     OT *out, const double *__restrict__ G, const double *__restrict__ factors, int64_t nplanes,
     const double *__restrict__ uvw, const double *__restrict__ freq, const WT *__restrict__ wt,
     const uint8_t *__restrict__ flag, int64_t n_u, int64_t n_v, double dl0, double dl1,
-    int64_t nt, int64_t nb, int64_t nchan, int64_t steps, int vec, int *err) {
-  const int64_t s = blockIdx.x * (int64_t)WT_THREADS + threadIdx.x;
-  if (s >= nb * nchan) return;
-  const int64_t b = s / nchan, c = s - b * nchan;
+    int64_t nt, int64_t nb, int64_t nchan, WeightWalk walk, int vec, int *err) {
+  const WeightPlace place(walk, nt, nb, nchan);
+  if (place.n <= 0) return;
+  const int64_t c = place.c;
   const double us0 = uv_scale(freq[c], dl0, n_u), us1 = uv_scale(freq[c], dl1, n_v);
   const double f0 = factors[c], f1 = factors[nplanes + c];
   const bool bad = isnan(f0) || isnan(f1);
   const double *plane = G + c * n_u * n_v;
   int64_t cell = -1;
   double gij = 0.0;
-  const int64_t t0 = blockIdx.y * steps, t1 = std::min(nt, t0 + steps);
-  for (int64_t t = t0; t < t1; t += WT_UNROLL) {
+  int64_t at_t = place.at;  // row of uvw
+  for (int left = place.n; left > 0; left -= WT_UNROLL, at_t += WT_UNROLL * nb) {
     double um[WT_UNROLL], vm[WT_UNROLL], dw[WT_UNROLL];
 #pragma unroll
     for (int k = 0; k < WT_UNROLL; ++k)
-      if (t + k < t1) {
-        const int64_t tb = (t + k) * nb + b;
+      if (k < left) {
+        const int64_t tb = at_t + k * nb;
         um[k] = uvw[3 * tb];
         vm[k] = uvw[3 * tb + 1];
         dw[k] = pol_avg_weight<NPOL>(wt, flag, tb * nchan + c);
       }
 #pragma unroll
     for (int k = 0; k < WT_UNROLL; ++k) {
-      if (t + k >= t1) continue;
+      if (k >= left) continue;
       double iw = 0.0;  // off-grid samples keep the zero the reference allocates
       long long ui, vi, uic, vic;
       if (scaled_cell(um[k], vm[k], us0, us1, n_u, n_v, ui, vi, uic, vic)) {
@@ -263,7 +293,7 @@ __global__ void __launch_bounds__(WT_THREADS, 4) k_briggs_apply(
           }
         }
       }
-      OT *o = out + (((t + k) * nb + b) * nchan + c) * NPOL;
+      OT *o = out + ((at_t + k * nb) * nchan + c) * NPOL;
       const OT v = (OT)iw;
       if (NPOL > 1 && vec) {  // out is 16-byte aligned
         using V = typename PairOf<OT>::type;
@@ -339,12 +369,11 @@ int av_weight_density(double *density, double *sum_weight, const double *uvw,
   AV_CHECK_ARG(n_u > 0 && n_v > 0 && nt >= 0 && nb >= 0 && nchan >= 0,
                "av_weight_density: bad shape");
   if (nt * nb * nchan == 0) return AV_OK;
-  int64_t steps = 0;
-  const dim3 grid = weight_walk(nt, nb * nchan, steps);
+  const WeightWalk walk = weight_walk(nt, nb, nchan);
   auto run = [&](auto pol, const auto *w) {
-    k_weight_density<decltype(pol)::value><<<grid, WT_THREADS, 0, as_stream(stream)>>>(
+    k_weight_density<decltype(pol)::value><<<walk.blocks, WT_THREADS, 0, as_stream(stream)>>>(
         density, sum_weight, uvw, freq, w, flag, n_u, n_v, delta_l, delta_m, nt, nb, nchan,
-        steps);
+        walk);
   };
   with_pols(npol, [&](auto pol) {
     if (wt_dtype == AV_F32) run(pol, (const float *)wt);
@@ -393,13 +422,12 @@ int av_briggs_apply(void *out, int out_dtype, const double *density, const doubl
   AV_CHECK_ARG(wt_dtype == AV_F32 || wt_dtype == AV_F64, "av_briggs_apply: weight dtype");
   AV_CHECK_ARG(npol == 1 || npol == 2 || npol == 4, "av_briggs_apply: npol must be 1, 2 or 4");
   if (nt * nb * nchan == 0) return AV_OK;
-  int64_t steps = 0;
-  const dim3 grid = weight_walk(nt, nb * nchan, steps);
+  const WeightWalk walk = weight_walk(nt, nb, nchan);
   const int vec = (((uintptr_t)out) & 15) == 0;
   auto run = [&](auto pol, auto *o, const auto *w) {
-    k_briggs_apply<decltype(pol)::value><<<grid, WT_THREADS, 0, as_stream(stream)>>>(
+    k_briggs_apply<decltype(pol)::value><<<walk.blocks, WT_THREADS, 0, as_stream(stream)>>>(
         o, density, factors, nchan, uvw, freq, w, flag, n_u, n_v, delta_l, delta_m, nt, nb, nchan,
-        steps, vec, err_flag);
+        walk, vec, err_flag);
   };
   with_pols(npol, [&](auto pol) {
     if (out_dtype == AV_F64 && wt_dtype == AV_F64) run(pol, (double *)out, (const double *)wt);
