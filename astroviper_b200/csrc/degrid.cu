@@ -219,13 +219,15 @@ struct DSmem {
 // FP32 taps of offset o - 128 and their FP64 sum rs[o] (RECIPROCAL: 1 / sum,
 // infinite for a zero sum).  The sum is the rounded taps' own, so a constant
 // grid degrids to itself: with the unrounded taps' sum the error of cubes of
-// 0.9M samples against FP64 is 4 % larger.
+// 0.9M samples against FP64 is 4 % larger.  Where rounding changes the sum by
+// more than its own relative error (taps that cancel, or leave FP32's range),
+// the unrounded taps' sum counts: it says which samples have no norm.
 template <int S, int RW, bool RECIPROCAL>
 __device__ void build_tap_tables_d(float *tab, double *rs, const double *cgk, int cgk_len,
                                    int os) {
   for (int o = threadIdx.x; o < 256; o += blockDim.x) {
     int off = o - 128;
-    double s = 0.0;
+    double s = 0.0, exact = 0.0;
 #pragma unroll
     for (int i = 0; i < RW; ++i) {
       double v = 0.0;
@@ -237,7 +239,9 @@ __device__ void build_tap_tables_d(float *tab, double *rs, const double *cgk, in
       const float t = (float)v;
       tab[o * RW + i] = t;
       s += (double)t;
+      exact += v;
     }
+    if (!(fabs(s - exact) <= 1e-6 * fabs(exact))) s = exact;
     rs[o] = RECIPROCAL ? 1.0 / s : s;
   }
 }
