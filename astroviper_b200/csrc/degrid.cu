@@ -438,6 +438,16 @@ __device__ __forceinline__ void stage_subgrid(const DegridArgs &d, float2 *sub, 
   }
 }
 
+// CTAs per SM that k_degrid_tiled's registers are to leave room for; 0 leaves
+// it to the compiler, which for the variants below takes more registers than
+// hide latency, or spills to save some.
+template <int S, int NPG, bool STORE>
+constexpr int degrid_min_ctas() {
+  if (NPG == 1) return STORE || (S != 7 && S != 9) ? 4 : 0;
+  if (NPG == 2) return (STORE ? S == 6 : S >= 8) ? 3 : 0;
+  return 0;
+}
+
 // STORE (complex64 store mode without phase): reciprocals of the taps' sums in
 // the table, so no sample needs an FP64 divide; flags read at the start of a
 // step, their latency behind the footprint's sums; one store per sample:
@@ -446,7 +456,7 @@ __device__ __forceinline__ void stage_subgrid(const DegridArgs &d, float2 *sub, 
 // (Taps divided by their sums and no scaling at all: 81 and 91 us, but a
 // norm that is rounded to FP32 with them.)
 template <int S, int NPG, bool STORE>
-__global__ void __launch_bounds__(DT_THREADS) k_degrid_tiled(TiledDegridArgs a) {
+__global__ void __launch_bounds__(DT_THREADS, degrid_min_ctas<S, NPG, STORE>()) k_degrid_tiled(TiledDegridArgs a) {
   using M = DSmem<S, NPG>;
   constexpr int W = M::W, RW = M::RW;
   extern __shared__ __align__(16) unsigned char smem[];
