@@ -824,6 +824,22 @@ def mosaic_runs_ok(n_cf, cu, cv, max_support, oversampling, npol):
             and rows * max_support ** 2 <= 4 * n_cf * cu * cv + (1 << 20))
 
 
+def _mosaic_taps_pay(n_cf, max_support, oversampling, samples, npol):
+    """Whether the kernel with the footprint in registers saves more over the
+    tiled one than gathering its tap table costs, in microseconds: 0.6 to 1.26
+    ns a row (supports 0 to 11; one row per function and kernel offset) against
+    0.25 ns and 0.055 more per cell of the support for a correlation, and what
+    the tiled kernel's first thousand samples of a CTA take.  Over 1184 calls
+    (1404 to 806400 samples, supports 3-11, oversampling 4-20, 1 to 2400
+    functions) the side taken is never slower than the tiled kernel by more
+    than 3 %, and in 39 of them the slower side (by up to 1.46 times); without
+    this rule the kernel lost to the tiled one in 99, by up to 4.7 times."""
+    gather = (0.6 + 0.06 * max_support) * 1e-3 * n_cf * (oversampling + 1) ** 2
+    saved = (20.0 + 0.8 * max_support ** 2 * npol * min(1.0, samples / 1024.0)
+             + (0.25 + 0.055 * max_support) * 1e-3 * samples * npol)
+    return gather <= saved
+
+
 def mosaic_grid(grid, sum_weight, do_psf, vis, weight, uvw, freq, chan_map, pol_map, cfb_map,
                 cfc_map, cfp_map, cf, support, n_uv, delta_lm, oversampling, aperture=False,
                 tiled=None):
@@ -865,7 +881,8 @@ def mosaic_grid(grid, sum_weight, do_psf, vis, weight, uvw, freq, chan_map, pol_
                                      nb, nchan, n_img_chan, wptr, wbytes, stream_ptr()),
           "av_mosaic_tiled_plan")
     n_cf = n_cfb * n_cfc * n_cfp
-    if mosaic_runs_ok(n_cf, cu, cv, max_sup, os_u, npol):
+    if (mosaic_runs_ok(n_cf, cu, cv, max_sup, os_u, npol)
+            and _mosaic_taps_pay(n_cf, max_sup, os_u, nt * nb * nchan, npol)):
         tab = _scratch(lib().av_mosaic_taps_size(n_cf, max_sup, os_u))
         if tab is not None:
             check(lib().av_mosaic_runs_execute(*args, wptr, wbytes, tab[1], tab[2],

@@ -10,3 +10,14 @@ import pytest
 def test_route(args, want):
     from astroviper_b200 import _kernels as K
     assert K.mosaic_runs_ok(*args) is want
+
+
+@pytest.mark.parametrize("args,want", [
+    # a mosaic's few functions, whatever the samples
+    ((6, 7, 4, 500, 2), True), ((6, 7, 4, 1_000_000, 2), True), ((6, 11, 20, 1404, 4), True),
+    # a table of a million rows: only for many samples
+    ((2400, 7, 20, 28_080, 1), False), ((2400, 11, 20, 1404, 2), False),
+    ((2400, 7, 20, 10_000_000, 2), True)])
+def test_tap_table_against_samples(args, want):
+    from astroviper_b200 import _kernels as K
+    assert K._mosaic_taps_pay(*args) is want
