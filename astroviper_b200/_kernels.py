@@ -71,13 +71,16 @@ def on_device(x, dtype=None):
 
 
 _NP_OF = {torch.float64: np.float64, torch.int32: np.int32}
+# real numbers in native byte order, up to 8 bytes
+_PACKED_TYPES = frozenset(np.dtype(c) for c in "?bBhHiIlLqQefd")
 
 
 def _packable(x):
     """Whether upload packs x: an array of real numbers that torch takes too
     (not one of strings, objects, dates, foreign bytes or negative strides)."""
-    return (isinstance(x, np.ndarray) and x.dtype.kind in "fiub" and x.dtype.itemsize <= 8
-            and x.dtype.isnative and min(x.strides, default=0) >= 0)
+    if not isinstance(x, np.ndarray) or x.dtype not in _PACKED_TYPES:
+        return False
+    return x.strides[0] >= 0 if x.ndim == 1 else min(x.strides, default=0) >= 0
 
 
 def upload(*items):
@@ -95,7 +98,9 @@ def upload(*items):
         if capturing or not _packable(x):
             out[i] = on_device(x, dt)
         else:
-            a = np.ascontiguousarray(x, dtype=_NP_OF[dt]).reshape(x.shape)
+            a = np.ascontiguousarray(x, dtype=_NP_OF[dt])
+            if not x.ndim:  # ascontiguousarray makes it one element
+                a = a.reshape(())
             pack.append((i, a, size))
             size += (a.nbytes + 15) & ~15
     if size == 0:
