@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <deque>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -113,8 +114,8 @@ __global__ void k_ishift_in(const IT *in, CT *buf, int64_t nplanes, int64_t nx, 
   buf[k] = o;
 }
 
-// The kernels around the real transforms.  A block takes IMG_COLS columns of
-// IMG_ROWS rows of one plane (grid: column tiles, row groups, planes), so a
+// The kernels around the real transforms.  A block takes 128 columns of 16
+// rows of one plane (grid: column tiles, row groups, planes), so a
 // thread evaluates the grid correction's factor of its column once and the
 // block the factors of its rows once: an evaluation per pixel, a long chain
 // of FP64 operations and divides, had made the epilogue of four 2048^2 images
@@ -126,23 +127,52 @@ __global__ void k_ishift_in(const IT *in, CT *buf, int64_t nplanes, int64_t nx, 
 // gather 95 -> 62 us and cuFFT 289 -> 175 us for four 2048^2 planes, whole
 // images 932 -> 302 us.  Batches of planes small enough to stay in L2 between
 // the passes gained nothing (374 us: cuFFT is bound by its FP64 work there).
-constexpr int IMG_COLS = 128, IMG_ROWS = 16, IMG_UNROLL = 8;
+// A plane whose blocks would leave SMs idle takes 4 rows to a block (257^2:
+// 33 us -> 31, 512^2 25 -> 23), and one of up to 64 columns, whose rows would
+// leave most threads idle, eight groups of 4 rows side by side (20,000 x 20:
+// 39 -> 32 us, 100,000 x 2 74 -> 50).  Single planes of odd size below 500^2
+// stay slower than with complex transforms (257^2: 23 us), for the library's
+// real ones: hidden behind the call's host work.
+constexpr int IMG_THREADS = 128, IMG_UNROLL = 8;
 
-static dim3 img_grid(int64_t nplanes, int64_t rows, int64_t cols) {
-  return dim3((unsigned)((cols + IMG_COLS - 1) / IMG_COLS),
-              (unsigned)std::min<int64_t>((rows + IMG_ROWS - 1) / IMG_ROWS, 65535),
-              (unsigned)std::min<int64_t>(nplanes, 65535));
-}
+// LANES groups of ROWS rows side by side, THREADS / LANES columns wide.
+template <int LANES_, int ROWS_>
+struct ImgBlock {
+  static constexpr int LANES = LANES_, ROWS = ROWS_, COLS = IMG_THREADS / LANES;
+  static constexpr int UNROLL = ROWS < IMG_UNROLL ? ROWS : IMG_UNROLL;
+  static_assert(COLS >= ROWS, "a group's threads set up its rows");
+  static dim3 grid(int64_t nplanes, int64_t rows, int64_t cols) {
+    return dim3((unsigned)((cols + COLS - 1) / COLS),
+                (unsigned)std::min<int64_t>((rows + LANES * ROWS - 1) / (LANES * ROWS), 65535),
+                (unsigned)std::min<int64_t>(nplanes, 65535));
+  }
+  // For the passes with the grid correction: two planes to a block where that
+  // leaves 16 blocks per SM, so a factor serves twice the pixels (four 2048^2
+  // images 68 -> 61 us).
+  static dim3 pixel_grid(int64_t nplanes, int64_t nx, int64_t ny) {
+    dim3 g = grid(nplanes, nx, ny);
+    const int64_t pairs = (nplanes + 1) / 2;
+    if (pairs <= 65535 && (int64_t)g.x * g.y * pairs >= (int64_t)sm_count() * 16)
+      g.z = (unsigned)pairs;
+    return g;
+  }
+  static __device__ __forceinline__ int place() {  // in the group
+    return LANES == 1 ? threadIdx.x : threadIdx.x % COLS;
+  }
+  static __device__ __forceinline__ int64_t col() {
+    return blockIdx.x * (int64_t)COLS + place();
+  }
+  static __device__ __forceinline__ int lane() { return LANES == 1 ? 0 : threadIdx.x / COLS; }
+};
 
-// For the passes with the grid correction: two planes to a block where that
-// leaves 16 blocks per SM, so a factor serves twice the pixels (four 2048^2
-// images 68 -> 61 us).
-static dim3 pixel_grid(int64_t nplanes, int64_t nx, int64_t ny) {
-  dim3 g = img_grid(nplanes, nx, ny);
-  const int64_t pairs = (nplanes + 1) / 2;
-  if (pairs <= 65535 && (int64_t)g.x * g.y * pairs >= (int64_t)sm_count() * 16)
-    g.z = (unsigned)pairs;
-  return g;
+// f(the block's shape) for planes of rows x cols.
+template <typename F>
+static void with_img_block(int64_t nplanes, int64_t rows, int64_t cols, F f) {
+  using Wide = ImgBlock<1, 16>;
+  if (cols <= 64) return f(ImgBlock<8, 4>());
+  const dim3 g = Wide::grid(nplanes, rows, cols);
+  if ((int64_t)g.x * g.y * g.z < 2 * (int64_t)sm_count()) return f(ImgBlock<1, 4>());
+  f(Wide());
 }
 
 // i + s for 0 <= i < n, 0 <= s <= n, modulo n.
@@ -186,46 +216,50 @@ __device__ __forceinline__ double quotient_by(double v, double d, double r) {
   return fma(fma(-q, d, v), r, q);
 }
 
-// Carries every pixel of this block's share from f.in to f.out, IMG_UNROLL
+// Carries every pixel of this block's share from f.in to f.out, B::UNROLL
 // rows at a time, with the grid correction's factors and their reciprocals (1
 // without apply_corr).  The rows' wrapped offsets are worked out once for the
 // block's planes: 64-bit index arithmetic per pixel had made the pass issue
 // bound.
-template <typename F>
+template <typename B, typename F>
 __device__ __forceinline__ void for_pixels(int64_t nplanes, int64_t nx, int64_t ny,
                                            int apply_corr, F f) {
-  __shared__ double2 s_gx[IMG_ROWS];
-  __shared__ int64_t s_in[IMG_ROWS], s_out[IMG_ROWS];
-  const int64_t j = blockIdx.x * (int64_t)IMG_COLS + threadIdx.x;
+  __shared__ double2 sh_gx[B::LANES][B::ROWS];
+  __shared__ int64_t sh_in[B::LANES][B::ROWS], sh_out[B::LANES][B::ROWS];
+  double2 *s_gx = sh_gx[B::lane()];
+  int64_t *s_in = sh_in[B::lane()], *s_out = sh_out[B::lane()];
+  const int t = B::place();
+  const int64_t j = B::col();
   double2 gy = make_double2(1.0, 1.0);
   if (apply_corr && j < ny) {
     gy.x = corr_factor(j, ny);
     gy.y = 1.0 / gy.x;
   }
-  for (int64_t i0 = blockIdx.y * (int64_t)IMG_ROWS; i0 < nx;
-       i0 += gridDim.y * (int64_t)IMG_ROWS) {
+  constexpr int64_t STEP = B::LANES * B::ROWS;
+  for (int64_t first = blockIdx.y * STEP; first < nx; first += gridDim.y * STEP) {
+    const int64_t i0 = first + B::lane() * B::ROWS;
     __syncthreads();
-    if (threadIdx.x < IMG_ROWS && i0 + threadIdx.x < nx) {
-      const int64_t i = i0 + threadIdx.x;
+    if (t < B::ROWS && i0 + t < nx) {
+      const int64_t i = i0 + t;
       const double g = apply_corr ? corr_factor(i, nx) : 1.0;
-      s_gx[threadIdx.x] = make_double2(g, 1.0 / g);
-      s_in[threadIdx.x] = f.row_in(i);
-      s_out[threadIdx.x] = f.row_out(i);
+      s_gx[t] = make_double2(g, 1.0 / g);
+      s_in[t] = f.row_in(i);
+      s_out[t] = f.row_out(i);
     }
     __syncthreads();
     if (j >= ny) continue;
-    const int rows = (int)std::min<int64_t>(IMG_ROWS, nx - i0);
+    const int rows = (int)std::min<int64_t>(B::ROWS, nx - i0);  // below 1 past the image
     for (int64_t p = blockIdx.z; p < nplanes; p += gridDim.z) {
       const double sw = f.sumw ? f.sumw[p] : 1.0, rsw = reciprocal_for_quotient(sw);
       const auto *in = f.in + p * f.plane_in() + f.col_in(j);
       auto *out = f.out + p * f.plane_out() + f.col_out(j);
-      for (int r = 0; r < rows; r += IMG_UNROLL) {
-        double v[IMG_UNROLL];
+      for (int r = 0; r < rows; r += B::UNROLL) {
+        double v[B::UNROLL];
 #pragma unroll
-        for (int k = 0; k < IMG_UNROLL; ++k)
+        for (int k = 0; k < B::UNROLL; ++k)
           if (r + k < rows) v[k] = (double)in[s_in[r + k]];
 #pragma unroll
-        for (int k = 0; k < IMG_UNROLL; ++k)
+        for (int k = 0; k < B::UNROLL; ++k)
           if (r + k < rows) {
             const double2 gx = s_gx[r + k];
             if (apply_corr) v[k] = quotient(v[k], gx.x * gy.x, gx.y * gy.y);
@@ -240,30 +274,30 @@ __device__ __forceinline__ void for_pixels(int64_t nplanes, int64_t nx, int64_t 
 // Half spectrum of the Hermitian part of the ifftshifted grid:
 // buf[i, j] = (s[i, j] + conj(s[-i, -j])) / 2, j <= ny / 2, with
 // s[i, j] = grid[(i + nx/2) % nx, (j + ny/2) % ny].
-template <typename IT>
-__global__ void __launch_bounds__(IMG_COLS) k_herm_in(const IT *grid, double2 *buf,
-                                                      int64_t nplanes, int64_t nx, int64_t ny) {
+template <typename B, typename IT>
+__global__ void __launch_bounds__(IMG_THREADS) k_herm_in(const IT *grid, double2 *buf,
+                                                         int64_t nplanes, int64_t nx, int64_t ny) {
   const int64_t h = half_cols(ny);
-  const int64_t j = blockIdx.x * (int64_t)IMG_COLS + threadIdx.x;
+  const int64_t j = B::col();
   if (j >= h) return;
   const int64_t ja = wrap(j, ny / 2, ny);
   const int64_t jb = wrap(j == 0 ? 0 : ny - j, ny / 2, ny);
-  for (int64_t i0 = blockIdx.y * (int64_t)IMG_ROWS; i0 < nx;
-       i0 += gridDim.y * (int64_t)IMG_ROWS) {
-    const int rows = (int)std::min<int64_t>(IMG_ROWS, nx - i0);
+  constexpr int64_t STEP = B::LANES * B::ROWS;
+  for (int64_t i0 = blockIdx.y * STEP + B::lane() * B::ROWS; i0 < nx; i0 += gridDim.y * STEP) {
+    const int rows = (int)std::min<int64_t>(B::ROWS, nx - i0);
     for (int64_t p = blockIdx.z; p < nplanes; p += gridDim.z) {
       const IT *g = grid + p * nx * ny;
-      for (int r = 0; r < rows; r += IMG_UNROLL) {
-        IT a[IMG_UNROLL], b[IMG_UNROLL];
+      for (int r = 0; r < rows; r += B::UNROLL) {
+        IT a[B::UNROLL], b[B::UNROLL];
 #pragma unroll
-        for (int k = 0; k < IMG_UNROLL; ++k)
+        for (int k = 0; k < B::UNROLL; ++k)
           if (r + k < rows) {
             const int64_t i = i0 + r + k;
             a[k] = __ldcs(g + wrap(i, nx / 2, nx) * ny + ja);
             b[k] = __ldcs(g + wrap(i == 0 ? 0 : nx - i, nx / 2, nx) * ny + jb);
           }
 #pragma unroll
-        for (int k = 0; k < IMG_UNROLL; ++k)
+        for (int k = 0; k < B::UNROLL; ++k)
           if (r + k < rows)
             buf[(p * nx + i0 + r + k) * h + j] =
                 make_double2(0.5 * ((double)a[k].x + (double)b[k].x),
@@ -293,10 +327,10 @@ struct ImageEpilogue {
   __device__ void store(OT *at, double v) const { __stcs(at, (OT)v); }
 };
 
-template <typename OT>
-__global__ void __launch_bounds__(IMG_COLS) k_image_epilogue(ImageEpilogue<OT> f,
-                                                             int64_t nplanes) {
-  for_pixels(nplanes, f.nx, f.ny, f.apply_corr, f);
+template <typename B, typename OT>
+__global__ void __launch_bounds__(IMG_THREADS) k_image_epilogue(ImageEpilogue<OT> f,
+                                                                int64_t nplanes) {
+  for_pixels<B>(nplanes, f.nx, f.ny, f.apply_corr, f);
 }
 
 // ifftshift of a real image into the transform's real rows, divided by the
@@ -319,39 +353,39 @@ struct ImagePrologue {
   __device__ void store(double *at, double v) const { *at = v; }
 };
 
-template <typename IT>
-__global__ void __launch_bounds__(IMG_COLS) k_image_prologue(ImagePrologue<IT> f,
-                                                             int64_t nplanes) {
-  for_pixels(nplanes, f.nx, f.ny, f.apply_corr, f);
+template <typename B, typename IT>
+__global__ void __launch_bounds__(IMG_THREADS) k_image_prologue(ImagePrologue<IT> f,
+                                                                int64_t nplanes) {
+  for_pixels<B>(nplanes, f.nx, f.ny, f.apply_corr, f);
 }
 
 // fftshift of a half spectrum to a full grid: the other half is the
 // conjugate of the mirrored one.
-template <typename OT>
-__global__ void __launch_bounds__(IMG_COLS) k_herm_out(const double2 *buf, OT *grid,
-                                                       int64_t nplanes, int64_t nx,
-                                                       int64_t ny) {
+template <typename B, typename OT>
+__global__ void __launch_bounds__(IMG_THREADS) k_herm_out(const double2 *buf, OT *grid,
+                                                          int64_t nplanes, int64_t nx,
+                                                          int64_t ny) {
   const int64_t h = half_cols(ny);
-  const int64_t j = blockIdx.x * (int64_t)IMG_COLS + threadIdx.x;
+  const int64_t j = B::col();
   if (j >= ny) return;
   const int64_t sj = wrap(j, ny - ny / 2, ny);
   const bool mirror = sj >= h;
   const int64_t bj = mirror ? ny - sj : sj;
-  for (int64_t i0 = blockIdx.y * (int64_t)IMG_ROWS; i0 < nx;
-       i0 += gridDim.y * (int64_t)IMG_ROWS) {
-    const int rows = (int)std::min<int64_t>(IMG_ROWS, nx - i0);
+  constexpr int64_t STEP = B::LANES * B::ROWS;
+  for (int64_t i0 = blockIdx.y * STEP + B::lane() * B::ROWS; i0 < nx; i0 += gridDim.y * STEP) {
+    const int rows = (int)std::min<int64_t>(B::ROWS, nx - i0);
     for (int64_t p = blockIdx.z; p < nplanes; p += gridDim.z)
-      for (int r = 0; r < rows; r += IMG_UNROLL) {
-        double2 v[IMG_UNROLL];
+      for (int r = 0; r < rows; r += B::UNROLL) {
+        double2 v[B::UNROLL];
 #pragma unroll
-        for (int k = 0; k < IMG_UNROLL; ++k)
+        for (int k = 0; k < B::UNROLL; ++k)
           if (r + k < rows) {
             int64_t si = wrap(i0 + r + k, nx - nx / 2, nx);
             if (mirror && si != 0) si = nx - si;
             v[k] = buf[(p * nx + si) * h + bj];
           }
 #pragma unroll
-        for (int k = 0; k < IMG_UNROLL; ++k)
+        for (int k = 0; k < B::UNROLL; ++k)
           if (r + k < rows) {
             OT o;
             o.x = v[k].x;
@@ -467,25 +501,28 @@ int av_grid_to_image(const void *grid, int grid_dtype, const double *sum_weight,
   double2 *buf = ws.take<double2>(bufb / sizeof(double2));
   void *work = ws.take<char>(workb > 0 ? workb : 1);
   cudaStream_t st = as_stream(stream);
-  const dim3 half = img_grid(nplanes, nx, half_cols(ny)),
-             full = pixel_grid(nplanes, nx, ny);
-  if (grid_dtype == AV_C128)
-    k_herm_in<double2><<<half, IMG_COLS, 0, st>>>((const double2 *)grid, buf, nplanes,
-                                                  nx, ny);
-  else
-    k_herm_in<float2><<<half, IMG_COLS, 0, st>>>((const float2 *)grid, buf, nplanes, nx,
-                                                 ny);
+  with_img_block(nplanes, nx, half_cols(ny), [&](auto block) {
+    using B = decltype(block);
+    const dim3 g = B::grid(nplanes, nx, half_cols(ny));
+    if (grid_dtype == AV_C128)
+      k_herm_in<B><<<g, IMG_THREADS, 0, st>>>((const double2 *)grid, buf, nplanes, nx, ny);
+    else
+      k_herm_in<B><<<g, IMG_THREADS, 0, st>>>((const float2 *)grid, buf, nplanes, nx, ny);
+  });
   AV_LAUNCH_CHECK();
   rc = run_fft(buf, FFT_Z2D, nplanes, nx, ny, CUFFT_INVERSE, work, st);
   if (rc) return rc;
-  if (image_dtype == AV_F64)
-    k_image_epilogue<double><<<full, IMG_COLS, 0, st>>>(
-        ImageEpilogue<double>{(const double *)buf, (double *)image, sum_weight, nx, ny,
-                              apply_corr}, nplanes);
-  else
-    k_image_epilogue<float><<<full, IMG_COLS, 0, st>>>(
-        ImageEpilogue<float>{(const double *)buf, (float *)image, sum_weight, nx, ny,
-                             apply_corr}, nplanes);
+  with_img_block(nplanes, nx, ny, [&](auto block) {
+    using B = decltype(block);
+    const dim3 g = B::pixel_grid(nplanes, nx, ny);
+    auto run = [&](auto *out) {
+      using T = std::remove_pointer_t<decltype(out)>;
+      k_image_epilogue<B, T><<<g, IMG_THREADS, 0, st>>>(
+          ImageEpilogue<T>{(const double *)buf, out, sum_weight, nx, ny, apply_corr}, nplanes);
+    };
+    if (image_dtype == AV_F64) run((double *)image);
+    else run((float *)image);
+  });
   AV_LAUNCH_CHECK();
   return AV_OK;
 }
@@ -513,23 +550,28 @@ int av_image_to_grid(const void *image, int image_dtype, void *grid, int grid_dt
   double2 *buf = ws.take<double2>(bufb / sizeof(double2));
   void *work = ws.take<char>(workb > 0 ? workb : 1);
   cudaStream_t st = as_stream(stream);
-  const dim3 full = img_grid(nplanes, nx, ny), pixels = pixel_grid(nplanes, nx, ny);
-  if (image_dtype == AV_F64)
-    k_image_prologue<double><<<pixels, IMG_COLS, 0, st>>>(
-        ImagePrologue<double>{(const double *)image, (double *)buf, nullptr, nx, ny,
-                              apply_corr}, nplanes);
-  else
-    k_image_prologue<float><<<pixels, IMG_COLS, 0, st>>>(
-        ImagePrologue<float>{(const float *)image, (double *)buf, nullptr, nx, ny,
-                             apply_corr}, nplanes);
+  with_img_block(nplanes, nx, ny, [&](auto block) {
+    using B = decltype(block);
+    const dim3 g = B::pixel_grid(nplanes, nx, ny);
+    auto run = [&](const auto *in) {
+      using T = std::remove_const_t<std::remove_pointer_t<decltype(in)>>;
+      k_image_prologue<B, T><<<g, IMG_THREADS, 0, st>>>(
+          ImagePrologue<T>{in, (double *)buf, nullptr, nx, ny, apply_corr}, nplanes);
+    };
+    if (image_dtype == AV_F64) run((const double *)image);
+    else run((const float *)image);
+  });
   AV_LAUNCH_CHECK();
   rc = run_fft(buf, FFT_D2Z, nplanes, nx, ny, CUFFT_FORWARD, work, st);
   if (rc) return rc;
-  if (grid_dtype == AV_C128)
-    k_herm_out<double2><<<full, IMG_COLS, 0, st>>>(buf, (double2 *)grid, nplanes, nx,
-                                                   ny);
-  else
-    k_herm_out<float2><<<full, IMG_COLS, 0, st>>>(buf, (float2 *)grid, nplanes, nx, ny);
+  with_img_block(nplanes, nx, ny, [&](auto block) {
+    using B = decltype(block);
+    const dim3 g = B::grid(nplanes, nx, ny);
+    if (grid_dtype == AV_C128)
+      k_herm_out<B><<<g, IMG_THREADS, 0, st>>>(buf, (double2 *)grid, nplanes, nx, ny);
+    else
+      k_herm_out<B><<<g, IMG_THREADS, 0, st>>>(buf, (float2 *)grid, nplanes, nx, ny);
+  });
   AV_LAUNCH_CHECK();
   return AV_OK;
 }
