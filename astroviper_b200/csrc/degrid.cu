@@ -439,13 +439,18 @@ __device__ __forceinline__ void stage_subgrid(const DegridArgs &d, float2 *sub, 
 }
 
 // CTAs per SM that k_degrid_tiled's registers are to leave room for; 0 leaves
-// it to the compiler, which for the variants below takes more registers than
-// hide latency, or spills to save some.
+// it to the compiler, which elsewhere takes more registers than hide latency,
+// or spills to save some.  968k samples, cold, the compiler's choice, 3 and 4:
+// 1 polarisation, accumulated, support 4 58, 58, 54 us, 6 61, 60, 58, 8 64.5,
+// 61.5, 60.5, 9 62.5, 62.4, 65.6, stored, 9 50, 44, 44; 2, stored, support 3
+// 48, 42, 41, 5 48, 51, 50, 6 52, 48, 55, accumulated, 8 102, 93, 100.  Stored,
+// support 7, they are within 3 us there, and the compiler's choice is 1-8 us
+// faster in whole calls (100,800 samples of 2 polarisations, 4.2M of one).
 template <int S, int NPG, bool STORE>
 constexpr int degrid_min_ctas() {
-  if (NPG == 1) return STORE || (S != 7 && S != 9) ? 4 : 0;
-  if (NPG == 2) return (STORE ? S == 6 : S >= 8) ? 3 : 0;
-  return 0;
+  if (NPG > 2 || (S == 7 && STORE)) return 0;
+  if (NPG == 1) return S >= 8 ? 3 : 4;
+  return S <= 4 ? 4 : (S == 5 ? 0 : 3);
 }
 
 // STORE (complex64 store mode without phase): reciprocals of the taps' sums in
