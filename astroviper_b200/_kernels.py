@@ -98,23 +98,24 @@ def upload(*items):
         if capturing or not _packable(x):
             out[i] = on_device(x, dt)
         else:
-            a = np.ascontiguousarray(x, dtype=_NP_OF[dt])
-            if not x.ndim:  # ascontiguousarray makes it one element
-                a = a.reshape(())
-            pack.append((i, a, size))
-            size += (a.nbytes + 15) & ~15
+            pack.append((i, x, dt, size))
+            size += (x.size * dt.itemsize + 15) & ~15
     if size == 0:
-        for i, a, _ in pack:
-            out[i] = torch.empty(a.shape, dtype=items[i][1], device=device())
+        for i, x, dt, _ in pack:
+            out[i] = torch.empty(x.shape, dtype=dt, device=device())
         return out
-    dev = device()
     host = torch.empty(size, dtype=torch.uint8, pin_memory=True)
-    view = host.numpy()
-    for i, a, at in pack:
-        view[at:at + a.nbytes] = a.reshape(-1).view(np.uint8)
-    buf = host.to(dev, non_blocking=True)
-    for i, a, at in pack:
-        out[i] = buf[at:at + a.nbytes].view(items[i][1]).view(a.shape)
+    mem = host.numpy()
+    mem = {dt: mem.view(n) for dt, n in _NP_OF.items()}
+    for _, x, dt, at in pack:
+        at //= dt.itemsize
+        mem[dt][at:at + x.size] = x.reshape(-1)
+    buf = host.to(device(), non_blocking=True)
+    buf = {dt: buf.view(dt) for dt in _NP_OF}
+    for i, x, dt, at in pack:
+        at //= dt.itemsize
+        t = buf[dt][at:at + x.size]
+        out[i] = t if x.ndim == 1 else t.view(x.shape)
     return out
 
 
