@@ -993,8 +993,8 @@ static bool hogbom_reg(const HogArgs<float> &a, int grid, cudaStream_t st, int &
 
 // ------------------------------------------------------------------ maximg --
 // Minimum and maximum straight into out: a float's order is its bits' signed
-// order from 0 up and their reversed unsigned order below, so the blocks'
-// results meet in integer atomics and no scratch is needed.  (One CTA took
+// order from 0 up and their reversed unsigned order below (-0 below 0), so the
+// blocks' results meet in integer atomics and no scratch is needed.  (One CTA took
 // 389 us for 2048^2; 296 take 5.6.)
 template <typename T>
 struct OrderBits;
@@ -1013,7 +1013,6 @@ template <typename T>
 __device__ __forceinline__ void atomic_extreme(T *p, T v, bool want_max) {
   using S = typename OrderBits<T>::S;
   using U = typename OrderBits<T>::U;
-  v += (T)0;  // -0 counts as 0
   S s;
   memcpy(&s, &v, sizeof(T));
   if (want_max ? s >= 0 : s < 0) {
